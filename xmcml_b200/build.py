@@ -20,7 +20,7 @@ LIB = os.path.join(HERE, "libxmcml_b200.so")
 
 SOURCES = ["transport.cu", "batch.cu", "surrogate.cu", "weight_table.cu", "noalloc.cu", "bvh_gpu.cu", "sparse_maps.cu",
            "capi.cpp", "io.cpp", "bvh.cpp"]
-HEADERS = ["xmc_internal.h", "geom.cuh", "photon.cuh", "tc_gemm.cuh", "mlp_fused.cuh"]
+HEADERS = ["xmc_internal.h", "geom.cuh", "photon.cuh", "walk.cuh", "transport_tail.cuh", "tc_gemm.cuh", "mlp_fused.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

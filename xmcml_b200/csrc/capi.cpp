@@ -41,7 +41,7 @@ static void free_context(Context* c) {
                      c->d_tbin, c->d_ledger, c->d_counter, c->d_status, c->d_scatter, c->d_traj,
                      c->d_replay, c->d_replay_count, c->d_replay_ledger, c->d_cells, c->d_cell_z, c->d_cell_entries,
                      c->d_big, c->d_cancel, c->d_wtab, c->d_xlog, c->d_cell_runs, c->d_nz_counts, c->d_nz_offsets,
-                     c->d_nz_tmp, c->d_nz_idx, c->d_nz_val};
+                     c->d_nz_tmp, c->d_nz_idx, c->d_nz_val, c->d_tail};
     for (void* p : dbufs)
         if (p) cudaFree(p);
     void* hbufs[] = {c->h_cancel, c->h_absorb, c->h_det, c->h_tbin, c->h_ledger, c->h_status, c->h_maps,
@@ -566,12 +566,24 @@ static int create_from_image(const HostImage& img, Context** out) {
     if (occ <= 0) return bail(fail(XMC_ERR_DEVICE, "transport kernel cannot be resident with this block size / shared memory"));
     c->blocks_per_sm = opt.blocks_per_sm > 0 ? std::min(opt.blocks_per_sm, occ) : occ;
     c->grid = c->num_sms * c->blocks_per_sm;
+    // tail kernel: the list holds what every warp of the transport grid may hand over
+    int tail_occ = 0, tail_photons = 0;
+    CK(tail_occupancy(kp, &c->tail_smem, &tail_occ, &tail_photons));
+    if (tail_occ > 0) {
+        c->tail_grid = c->num_sms * tail_occ;
+        CK(cudaMalloc(&c->d_tail, 256 + sizeof(TailPhoton) * (size_t)c->grid * (c->block / 32) * kTailLanes));
+        kp.tail_count = (unsigned*)c->d_tail;
+        kp.tail_next = kp.tail_count + 1;
+        kp.tail = (TailPhoton*)((unsigned char*)c->d_tail + 256);
+    }
     if ((opt.flags & XMC_DETECTOR_TRAJ) && opt.trajectory_log >= 0) {
-        // crossing log: one row per resident thread, reused photon after photon
+        // crossing log: one row per resident thread (and per photon that the tail kernel walks at a time),
+        // reused photon after photon
         // 4,096 entries: on the height field no detected photon overflows it (1,024 left 0.2 % of them
         // to the replay pass, whose longest walk added ~30 ms to a 1e7-photon run)
         const unsigned cap = opt.trajectory_log > 0 ? (unsigned)opt.trajectory_log : 4096u;
-        CK(cudaMalloc(&c->d_xlog, sizeof(unsigned) * (size_t)c->grid * c->block * cap));
+        const size_t rows = std::max((size_t)c->grid * c->block, (size_t)c->tail_grid * tail_photons);
+        CK(cudaMalloc(&c->d_xlog, sizeof(unsigned) * rows * cap));
         kp.xlog = (unsigned*)c->d_xlog;
         kp.xlog_cap = cap;
     }

@@ -63,12 +63,11 @@ __device__ __forceinline__ float fresnel_reflectance(float ni, float nt, float c
     return 0.5f * sd * sd * (cd * cd + cs * cs) / (ss * ss * cd * cd);
 }
 
-// GetNewPhotonDirection / ComputeCosineTheta (mcml_kernel.cpp:442-495): Henyey-Greenstein cos(theta)
-// from u1 by the inverse CDF (hg_* = 1 - g^2, 1 + g^2, 1 / 2g, 1 - g, 2g; isotropic when hg_e == 0),
-// azimuth 2 pi u2, and the rotation of (dx, dy, dz) with the near-vertical special case.
-__device__ __forceinline__ void hg_spin(float hg_a, float hg_b, float hg_c, float hg_d, float hg_e, float u1, float u2,
-                                        float& dx, float& dy, float& dz) {
-    float cost;
+// Deflection of an interaction (ComputeCosineTheta, mcml_kernel.cpp:442-463): Henyey-Greenstein
+// cos(theta) from u1 by the inverse CDF (hg_* = 1 - g^2, 1 + g^2, 1 / 2g, 1 - g, 2g; isotropic when
+// hg_e == 0) and sin(theta); sine and cosine of the azimuth 2 pi u2. It does not depend on the direction.
+__device__ __forceinline__ void hg_angles(float hg_a, float hg_b, float hg_c, float hg_d, float hg_e, float u1, float u2,
+                                          float& cost, float& sint, float& sp, float& cp) {
     if (hg_e != 0.0f) {
         const float t = hg_a / (hg_d + hg_e * u1);
         cost = (hg_b - t * t) * hg_c;
@@ -76,11 +75,15 @@ __device__ __forceinline__ void hg_spin(float hg_a, float hg_b, float hg_c, floa
         cost = 2.0f * u1 - 1.0f;
     }
     cost = fminf(1.0f, fmaxf(-1.0f, cost));
-    const float sint = sqrtf(fmaxf(0.0f, 1.0f - cost * cost));
+    sint = sqrtf(fmaxf(0.0f, 1.0f - cost * cost));
     float a = u2;
     a = a > 0.5f ? a - 1.0f : a;  // same angle as 2*pi*u, reduced to [-pi, pi]
-    float sp, cp;
     __sincosf(6.283185307179586f * a, &sp, &cp);
+}
+
+// GetNewPhotonDirection (mcml_kernel.cpp:464-495): rotation of (dx, dy, dz) by these angles, with the
+// near-vertical special case.
+__device__ __forceinline__ void hg_rotate(float cost, float sint, float sp, float cp, float& dx, float& dy, float& dz) {
     const float ux = dx, uy = dy, uz = dz;
     const float rho2 = ux * ux + uy * uy;
     float nx, ny, nz;
@@ -99,6 +102,13 @@ __device__ __forceinline__ void hg_spin(float hg_a, float hg_b, float hg_c, floa
     dx = nx * on;
     dy = ny * on;
     dz = nz * on;
+}
+
+__device__ __forceinline__ void hg_spin(float hg_a, float hg_b, float hg_c, float hg_d, float hg_e, float u1, float u2,
+                                        float& dx, float& dy, float& dz) {
+    float cost, sint, sp, cp;
+    hg_angles(hg_a, hg_b, hg_c, hg_d, hg_e, u1, u2, cost, sint, sp, cp);
+    hg_rotate(cost, sint, sp, cp, dx, dy, dz);
 }
 #endif
 

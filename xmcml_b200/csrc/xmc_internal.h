@@ -114,6 +114,26 @@ struct WarpQuery {
     unsigned char owner[kWarpQueryCells];
 };
 
+// A warp of the transport kernel hands its photons over to the tail kernel once no ids are left and at
+// most this many of its lanes hold a photon.
+constexpr int kTailLanes = 8;
+
+// A photon on its way from the transport kernel to the tail kernel: its state, and the row and length of
+// its crossing log.
+struct TailPhoton {
+    float px, py, pz, dx, dy, dz;
+    float time, trange, orange, tmin;
+    unsigned long long w, pid;
+    int layer, excl, rdet;
+    uint32_t visited, iter, xrow, xn;
+
+    template <class Ph>
+    __host__ __device__ static TailPhoton of(const Ph& p, uint32_t xrow, uint32_t xn) {
+        return {p.px, p.py, p.pz, p.dx, p.dy, p.dz, p.time, p.trange, p.orange, p.tmin, p.w, p.pid,
+                p.layer, p.excl, p.rdet, p.visited, p.iter, xrow, xn};
+    }
+};
+
 // z-intervals occupied by triangles (merged, padded, sorted): a step whose z-range lies strictly
 // inside a gap between them cannot cross any surface, so its ray query is skipped.
 constexpr int kMaxZSlabs = 24;
@@ -187,6 +207,11 @@ struct KParams {
     unsigned long long* tbin;     // [n_dets * n_time * 4]
     unsigned long long* ledger;   // [kLedgerSlots]
     unsigned long long* counter;  // photon id dispenser
+    // the photons that a run's last warps hand over to the tail kernel (null: none are)
+    TailPhoton* tail;             // [warps of the grid * kTailLanes]
+    unsigned* tail_count;         // photons listed
+    unsigned* tail_next;          // the tail kernel's dispenser of them
+    int tail_direct;              // tail kernel: takes its photons from the id dispenser instead of the list
     const volatile int* cancel;   // device cancel flag, written by xmc_cancel from another stream (may be null)
     int* status;                  // device status word: bit0 budget hit, bit1 cancelled
     // biasing (InputInfo.useBiasing): attractive point and weight-integral tables
@@ -209,6 +234,8 @@ struct Context {
     int grid_size = 0, n_dets = 0, n_time = 0;
     size_t smem_bytes = 0;
     int block = 256, blocks_per_sm = 0, num_sms = 0, grid = 0;
+    int tail_grid = 0;        // blocks of the tail kernel (0: not used)
+    size_t tail_smem = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     // device buffers
@@ -221,6 +248,7 @@ struct Context {
     cudaStream_t cancel_stream = nullptr;
     void* d_scatter = nullptr; void* d_traj = nullptr; void* d_replay = nullptr; void* d_replay_count = nullptr;
     void* d_replay_ledger = nullptr;
+    void* d_tail = nullptr;     // photons handed over to the tail kernel
     void* d_xlog = nullptr;     // crossing log of the trajectory maps
     unsigned long long replay_cap = 0;
     unsigned long long last_replayed = 0;  // photons the last run walked again (crossing log overflow)
@@ -314,6 +342,9 @@ cudaError_t sparse_maps_write(const unsigned long long* maps, size_t cells, int 
                               unsigned* idx, unsigned long long* val, cudaStream_t st);
 // transport.cu: occupancy of the kernel for a block size and dynamic shared memory.
 cudaError_t transport_occupancy(int block, size_t smem, int* blocks_per_sm, bool bias = false);
+// transport.cu: dynamic shared memory and resident blocks per SM of the tail kernel (sets its limit), and
+// the photons that one block walks at a time.
+cudaError_t tail_occupancy(const KParams& kp, size_t* smem, int* blocks_per_sm, int* photons_per_block);
 // transport.cu: Philox blocks computed on the device (self test).
 cudaError_t device_philox(uint32_t key0, uint32_t key1, uint64_t pid, uint32_t n, uint32_t* host_out);
 
