@@ -58,10 +58,16 @@ __device__ __forceinline__ float fresnel_reflectance(float ni, float nt, float c
     const float st = ni * si / nt;
     if (st >= 1.0f) return 1.0f;
     const float ct = sqrtf(1.0f - st * st);
-    const float cs = ci * ct - si * st, cd = ci * ct + si * st;
-    const float ss = si * ct + ci * st, sd = si * ct - ci * st;
-    return 0.5f * sd * sd * (cd * cd + cs * cs) / (ss * ss * cd * cd);
+    // Which product of each sum is rounded on its own is written out: left to the compiler it differs from
+    // kernel to kernel with the registers at hand, and a photon in ten million then takes the other branch.
+    const float pc = __fmul_rn(si, st), ps = __fmul_rn(si, ct);
+    const float cs = __fmaf_rn(ci, ct, -pc), cd = __fmaf_rn(ci, ct, pc);
+    const float ss = __fmaf_rn(ci, st, ps), sd = __fmaf_rn(-ci, st, ps);
+    return 0.5f * sd * sd * __fmaf_rn(cd, cd, __fmul_rn(cs, cs)) / (ss * ss * cd * cd);
 }
+
+// sqrt(x^2 + y^2) with the rounding written out, for the same reason.
+__device__ __forceinline__ float radius_xy(float x, float y) { return sqrtf(__fmaf_rn(x, x, __fmul_rn(y, y))); }
 
 // Deflection of an interaction (ComputeCosineTheta, mcml_kernel.cpp:442-463): Henyey-Greenstein
 // cos(theta) from u1 by the inverse CDF (hg_* = 1 - g^2, 1 + g^2, 1 / 2g, 1 - g, 2g; isotropic when

@@ -88,7 +88,7 @@ __device__ __forceinline__ void lat(unsigned long long* p, unsigned long long v)
 template <class Ph>
 __device__ int find_detector(const KParams& P, const DevDetector* __restrict__ s_det, const Ph& ph) {
     int det = -1;
-    const float l2 = ph.dx * ph.dx + ph.dy * ph.dy + ph.dz * ph.dz;
+    const float l2 = __fmaf_rn(ph.dz, ph.dz, __fmaf_rn(ph.dx, ph.dx, __fmul_rn(ph.dy, ph.dy)));
     const float ac = -ph.dz / l2;
     const int n_scan = P.rings_sorted ? P.n_cubes : P.n_dets;
     for (int i = 0; i < n_scan; ++i) {
@@ -99,7 +99,7 @@ __device__ int find_detector(const KParams& P, const DevDetector* __restrict__ s
                      ph.pz >= D.cz - D.hz && ph.pz < D.cz + D.hz;
         } else {
             const float ex = ph.px - D.cx, ey = ph.py - D.cy;
-            const float r = sqrtf(ex * ex + ey * ey);
+            const float r = radius_xy(ex, ey);
             inside = r >= D.hx && r < D.hy;
         }
         if (inside && (D.filter & ph.visited) && ac > D.cos_angle) {
@@ -112,7 +112,7 @@ __device__ int find_detector(const KParams& P, const DevDetector* __restrict__ s
         // the last one whose small radius is <= r, so the first match of the scan is this one
         const DevDetector* R = s_det + P.n_cubes;
         const float ex = ph.px - R[0].cx, ey = ph.py - R[0].cy;
-        const float r = sqrtf(ex * ex + ey * ey);
+        const float r = radius_xy(ex, ey);
         int lo = 0, hi = P.n_rings - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
