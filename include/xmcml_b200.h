@@ -443,7 +443,8 @@ int xmc_layout_offsets(int64_t* out, int max_count);
  * rays[6*i]) the nearest hit with tmin <= t <= tmax over the device image of `input` (distance,
  * surface id or -1, unit normal or NULL), through the xy cell grid where the kernel would use it
  * (bit 0 of `flags`) or the BVH only; bit 1 builds the image's BVH on GPU 0 (XMC_GPU_BVH) instead
- * of the host. Used by the test suites. */
+ * of the host. Bit 2: no query; t_out[i] is 1 where the clearance grid says that the segment of length
+ * tmax meets no triangle, else 0. Used by the test suites. */
 int xmc_debug_nearest(const InputInfo* input, int n_rays, const float* rays, float tmin, float tmax,
                       float* t_out, int* surf_out, float* normal_out, int flags);
 

@@ -448,6 +448,113 @@ int occupied_z_slabs(const GeomImage& g, float* lo, float* hi) {
     return (int)m.size();
 }
 
+void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std::vector<uint8_t>* clear) {
+    kp->clear_n[0] = kp->clear_n[1] = kp->clear_n[2] = 0;
+    clear->clear();
+    // big or horizontal triangles: their z-intervals say enough
+    std::vector<char> is_big((size_t)g.n_tris, 0);
+    GeomImage big;
+    for (size_t k = 0; k < grid.big.size(); k += 4) {
+        int t;
+        std::memcpy(&t, &grid.big[k].z, sizeof(t));
+        is_big[t] = 1;
+    }
+    for (int t = 0; t < g.n_tris; ++t) {
+        const float4* v = &g.tris[3 * (size_t)t];
+        if (!is_big[t] && !(v[0].z == v[1].z && v[0].z == v[2].z)) continue;
+        is_big[t] = 1;
+        ++big.n_tris;
+        for (int c = 0; c < 3; ++c) big.tris.push_back(v[c]);
+    }
+    if (big.n_tris >= g.n_tris) return;  // no others: the z-gaps say all there is
+    kp->n_zbig = occupied_z_slabs(big, kp->zbig_lo, kp->zbig_hi);
+    // padded boxes of the small triangles, and their bounds
+    auto box = [&](int t, float* lo, float* hi) {
+        const float4 a = g.tris[3 * (size_t)t], b = g.tris[3 * (size_t)t + 1], c = g.tris[3 * (size_t)t + 2];
+        const float v[3][3] = {{a.x, b.x, c.x}, {a.y, b.y, c.y}, {a.z, b.z, c.z}};
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = std::min(v[d][0], std::min(v[d][1], v[d][2]));
+            hi[d] = std::max(v[d][0], std::max(v[d][1], v[d][2]));
+            const float pad = 2e-5f * std::max(1.0f, std::max(std::fabs(lo[d]), std::fabs(hi[d])));
+            lo[d] -= pad;
+            hi[d] += pad;
+        }
+    };
+    float blo[3] = {INFINITY, INFINITY, INFINITY}, bhi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int t = 0; t < g.n_tris; ++t) {
+        if (is_big[t]) continue;
+        float lo[3], hi[3];
+        box(t, lo, hi);
+        for (int d = 0; d < 3; ++d) {
+            blo[d] = std::min(blo[d], lo[d]);
+            bhi[d] = std::max(bhi[d], hi[d]);
+        }
+    }
+    // cubic voxels where the bounds allow it, at least 8 along a thin axis (a height field's depth)
+    double len[3], volume = 1.0;
+    for (int d = 0; d < 3; ++d) {
+        len[d] = (double)bhi[d] - blo[d];
+        if (!(len[d] > 0.0) || !std::isfinite(len[d])) return;
+        volume *= len[d];
+    }
+    const double h = std::cbrt(volume / kClearanceVoxels);
+    int n[3];
+    for (int d = 0; d < 3; ++d) {
+        const int inner = (int)std::min((double)kClearanceAxis, std::max(8.0, std::ceil(len[d] / h)));
+        const double w = len[d] / inner;
+        n[d] = inner + 2 * kClearanceRim;
+        kp->small_lo[d] = blo[d];
+        kp->small_hi[d] = bhi[d];
+        kp->clear_o[d] = (float)(blo[d] - kClearanceRim * w);
+        kp->clear_i[d] = (float)(1.0 / w);
+    }
+    const size_t nx = (size_t)n[0], ny = (size_t)n[1], nz = (size_t)n[2];
+    try {
+        clear->assign(nx * ny * nz, (uint8_t)kMaxClearance);
+    } catch (const std::bad_alloc&) {
+        return;  // every segment is queried
+    }
+    uint8_t* const D = clear->data();
+    for (int t = 0; t < g.n_tris; ++t) {
+        if (is_big[t]) continue;
+        float lo[3], hi[3];
+        int i0[3], i1[3];
+        box(t, lo, hi);
+        for (int d = 0; d < 3; ++d) {  // the kernel's arithmetic: voxel indices are monotone in the coordinate
+            const float a = (lo[d] - kp->clear_o[d]) * kp->clear_i[d], b = (hi[d] - kp->clear_o[d]) * kp->clear_i[d];
+            i0[d] = std::max(0, std::min(n[d] - 1, (int)std::floor(a)));
+            i1[d] = std::max(0, std::min(n[d] - 1, (int)std::floor(b)));
+        }
+        for (int k = i0[2]; k <= i1[2]; ++k)
+            for (int j = i0[1]; j <= i1[1]; ++j)
+                std::memset(D + ((size_t)k * ny + j) * nx + i0[0], 0, (size_t)(i1[0] - i0[0] + 1));
+    }
+    // Chebyshev distance, one axis after the other: out[p] = min over q of max(|p - q|, in[q])
+    const size_t step[3] = {1, nx, nx * ny};
+    for (int d = 0; d < 3; ++d) {
+        const size_t lines = nx * ny * nz / n[d], s = step[d];
+        const int m = n[d];
+        const unsigned parts = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+        parallel_parts(parts, [&](unsigned part) {
+            uint8_t in[kClearanceAxis + 2 * kClearanceRim];
+            for (size_t l = lines * part / parts; l < lines * (part + 1) / parts; ++l) {
+                const size_t base = d == 0 ? l * nx : d == 1 ? (l / nx) * nx * ny + l % nx : l;
+                uint8_t* const line = D + base;
+                for (int p = 0; p < m; ++p) in[p] = line[(size_t)p * s];
+                for (int p = 0; p < m; ++p) {
+                    int best = in[p];
+                    for (int r = 1; r < best; ++r) {
+                        if (p - r >= 0) best = std::min(best, std::max(r, (int)in[p - r]));
+                        if (p + r < m) best = std::min(best, std::max(r, (int)in[p + r]));
+                    }
+                    line[(size_t)p * s] = (uint8_t)best;
+                }
+            }
+        });
+    }
+    for (int d = 0; d < 3; ++d) kp->clear_n[d] = n[d];
+}
+
 void build_xy_grid(const GeomImage& g, GridImage* out, int tris_per_cell) {
     const double tpc = std::max(1, tris_per_cell);
     *out = GridImage();

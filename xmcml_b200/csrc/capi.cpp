@@ -41,7 +41,7 @@ static void free_context(Context* c) {
                      c->d_tbin, c->d_ledger, c->d_counter, c->d_status, c->d_scatter, c->d_traj,
                      c->d_replay, c->d_replay_count, c->d_replay_ledger, c->d_cells, c->d_cell_z, c->d_cell_entries,
                      c->d_big, c->d_cancel, c->d_wtab, c->d_xlog, c->d_cell_runs, c->d_nz_counts, c->d_nz_offsets,
-                     c->d_nz_tmp, c->d_nz_idx, c->d_nz_val, c->d_tail};
+                     c->d_nz_tmp, c->d_nz_idx, c->d_nz_val, c->d_tail, c->d_clear};
     for (void* p : dbufs)
         if (p) cudaFree(p);
     void* hbufs[] = {c->h_cancel, c->h_absorb, c->h_det, c->h_tbin, c->h_ledger, c->h_status, c->h_maps,
@@ -306,6 +306,7 @@ int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img
         else build_xy_grid(geom, &img->grid, opt.grid_cell_tris > 0 ? opt.grid_cell_tris : 12);
     });
     kp.n_zocc = n_zocc;
+    build_clearance(geom, img->grid, &kp, &img->clear);
     kp.grid_x0 = img->grid.x0;
     kp.grid_y0 = img->grid.y0;
     kp.grid_icx = img->grid.icx;
@@ -506,11 +507,12 @@ static int create_from_image(const HostImage& img, Context** out) {
     CK(up(&c->d_cell_entries, img.grid.entries.data(), sizeof(float4) * img.grid.entries.size()));
     CK(up(&c->d_big, img.grid.big.data(), sizeof(float4) * img.grid.big.size()));
     CK(up(&c->d_cell_runs, img.grid.cell_runs.data(), sizeof(uint32_t) * img.grid.cell_runs.size()));
+    CK(up(&c->d_clear, img.clear.data(), img.clear.size()));
     if (img.kp.use_bias) {
         CK(up(&c->d_wtab, img.wtab.data(), sizeof(float) * img.wtab.size()));
         c->h2d_bytes += sizeof(float) * img.wtab.size();
     }
-    c->h2d_bytes += sizeof(uint2) * img.grid.cells.size() + sizeof(uint32_t) * img.grid.cell_runs.size() +
+    c->h2d_bytes += img.clear.size() + sizeof(uint2) * img.grid.cells.size() + sizeof(uint32_t) * img.grid.cell_runs.size() +
                     sizeof(float4) * (img.grid.cell_z.size() + img.grid.entries.size() + img.grid.big.size());
     const size_t absorb_b = sizeof(unsigned long long) * (size_t)c->grid_size;
     const size_t det_b = sizeof(unsigned long long) * 4 * (size_t)std::max(1, nd);
@@ -546,6 +548,7 @@ static int create_from_image(const HostImage& img, Context** out) {
     kp.cell_entries = (const float4*)c->d_cell_entries;
     kp.big = (const float4*)c->d_big;
     kp.cell_runs = (const uint32_t*)c->d_cell_runs;
+    kp.clear = (const uint8_t*)c->d_clear;
     kp.wtab = (const float*)c->d_wtab;
     kp.absorb = (unsigned long long*)c->d_absorb;
     kp.det = (unsigned long long*)c->d_det;

@@ -215,4 +215,32 @@ __host__ __device__ __forceinline__ bool grid_nearest(const uint2* __restrict__ 
     return true;
 }
 
+__host__ __device__ __forceinline__ int floor_to_int(float f) {
+#ifdef __CUDA_ARCH__
+    return __float2int_rd(f);
+#else
+    return (int)floorf(f);
+#endif
+}
+
+// True when the segment from (ox, oy, oz) to (ex, ey, ez) meets no triangle by the clearance grid (false says
+// nothing).
+__host__ __device__ __forceinline__ bool clear_segment(const KParams& P, float ox, float oy, float oz, float ex, float ey, float ez) {
+    if (P.clear_n[0] == 0) return false;
+    const float zl = fminf(oz, ez), zh = fmaxf(oz, ez);
+    for (int i = 0; i < P.n_zbig; ++i)
+        if (zl <= P.zbig_hi[i] && zh >= P.zbig_lo[i]) return false;
+    if (zl > P.small_hi[2] || zh < P.small_lo[2] || fminf(ox, ex) > P.small_hi[0] || fmaxf(ox, ex) < P.small_lo[0] ||
+        fminf(oy, ey) > P.small_hi[1] || fmaxf(oy, ey) < P.small_lo[1])
+        return true;
+    const int i0 = floor_to_int((ox - P.clear_o[0]) * P.clear_i[0]), i1 = floor_to_int((ex - P.clear_o[0]) * P.clear_i[0]);
+    const int j0 = floor_to_int((oy - P.clear_o[1]) * P.clear_i[1]), j1 = floor_to_int((ey - P.clear_o[1]) * P.clear_i[1]);
+    const int k0 = floor_to_int((oz - P.clear_o[2]) * P.clear_i[2]), k1 = floor_to_int((ez - P.clear_o[2]) * P.clear_i[2]);
+    if ((unsigned)i0 >= (unsigned)P.clear_n[0] || (unsigned)i1 >= (unsigned)P.clear_n[0] || (unsigned)j0 >= (unsigned)P.clear_n[1] ||
+        (unsigned)j1 >= (unsigned)P.clear_n[1] || (unsigned)k0 >= (unsigned)P.clear_n[2] || (unsigned)k1 >= (unsigned)P.clear_n[2])
+        return false;
+    const int d = (int)XMC_LDG(&P.clear[((size_t)k0 * P.clear_n[1] + j0) * P.clear_n[0] + i0]);
+    return max(max(abs(i1 - i0), abs(j1 - j0)), abs(k1 - k0)) < d;
+}
+
 }  // namespace xmc

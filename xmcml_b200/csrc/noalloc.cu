@@ -136,6 +136,7 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     kp.counter = reinterpret_cast<unsigned long long*>(scratch);
     kp.status = reinterpret_cast<int*>(scratch + sizeof(unsigned long long));
     kp.cancel = nullptr;
+    kp.clear_n[0] = 0;  // the clearance grid is not staged: every segment outside the z-gaps is queried
     kp.absorb = d_absorption;
     kp.det = d_detectors;
     kp.tbin = d_time_bins;

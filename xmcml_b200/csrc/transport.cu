@@ -10,6 +10,14 @@
 // which thread runs it and the tallies (64-bit fixed-point integer sums) are bit-identical for
 // every launch shape.
 //
+// A warp takes the free steps of its lanes (walk.cuh free_step: no ray query, the common case) in a loop of
+// their own, until P.query_batch lanes wait for a general step; then it takes those together: one
+// cooperative ray query, boundary optics, detection and deaths. Which lanes take a step together changes no
+// photon's path. B200, ps per step at 1e6 photons and more, every step general -> free steps apart, with
+// the clearance grid and the wider cell rectangles: planar stack with roulette 28.0 -> 18.7, height field
+// 34.7 -> 27.3, ellipsoid 87.6 -> 73.3, glass cover 46.4 -> 40.5. What bounds it now is instruction issue
+// (about 300 per free iteration of the warp, 17 of 32 lanes active on average) at 16 warps per SM.
+//
 // Per iteration (tissue layer): slot 0 step length; on a boundary hit slot 1 Fresnel test and
 // slot 2 roulette; on an interaction slot 1 HG cos(theta), slot 2 azimuth, slot 3 roulette.
 // Glass layer: slot 0 Fresnel test, slot 1 roulette. The photon-weight arithmetic is integer
@@ -31,7 +39,7 @@ namespace {
 // under the segment, culled by the cells' and entries' z-ranges; the nearest distance wins and equal
 // distances keep the lower triangle index. Instead of each lane walking its own cells and entries
 // (serial loops whose trip counts differ from lane to lane), the warp flattens the work:
-//   1. each querying lane's cell rectangle (at most kGridMaxCells cells; more: `fallback`, the lane
+//   1. each querying lane's cell rectangle (at most kWarpMaxCells cells; more: `fallback`, the lane
 //      uses the BVH) and its big-triangle candidates;
 //   2. all (lane, cell) pairs of the warp, 32 per round: cell header and z-intervals loaded by one
 //      lane each, cells whose intervals miss the segment dropped, the rest compacted into a list;
@@ -58,7 +66,7 @@ __device__ __forceinline__ void warp_grid_query(const KParams& P, WarpQuery& W, 
         const int i0 = max(0, (int)floorf(fx0)), i1 = min(P.grid_nx - 1, (int)floorf(fx1));
         const int j0 = max(0, (int)floorf(fy0)), j1 = min(P.grid_ny - 1, (int)floorf(fy1));
         const float zl = fminf(oz, ez), zh = fmaxf(oz, ez);
-        if (inside && (i1 - i0 + 1) * (j1 - j0 + 1) > kGridMaxCells) {
+        if (inside && (i1 - i0 + 1) * (j1 - j0 + 1) > kWarpMaxCells) {
             fallback = true;
         } else {
             for (int k = 0; k < P.n_big; ++k) {
@@ -145,49 +153,52 @@ __device__ __forceinline__ void warp_grid_query(const KParams& P, WarpQuery& W, 
             W.owner[pos] = (unsigned char)own;
         }
         nk += __popc(km);
-    }
-    __syncwarp();
-    // (lane, entry) pairs over the kept cells: exclusive scan of their entry counts
-    int n_ent = 0;
-    for (int base = 0; base < nk; base += 32) {
-        const int c = base + lane;
-        const int cnt = c < nk ? (int)W.cell[c].y : 0;
-        int inc = cnt;
+        if (nk + 32 <= kWarpQueryCells && base + 32 < n_pairs) continue;
+        __syncwarp();
+        // (lane, entry) pairs over the kept cells: exclusive scan of their entry counts
+        int n_ent = 0;
+        for (int base = 0; base < nk; base += 32) {
+            const int c = base + lane;
+            const int cnt = c < nk ? (int)W.cell[c].y : 0;
+            int inc = cnt;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(FULL, inc, o);
-            if (lane >= o) inc += v;
-        }
-        if (c < nk) W.eoff[c] = n_ent + inc - cnt;
-        n_ent += __shfl_sync(FULL, inc, 31);
-    }
-    __syncwarp();
-    for (int base = 0; base < n_ent; base += 32) {
-        const int k = base + lane;
-        if (k < n_ent) {
-            int lo = 0, hi = nk - 1;  // the entry's cell: the last kept cell whose offset is <= k
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (W.eoff[mid] <= k) lo = mid;
-                else hi = mid - 1;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += v;
             }
-            const int own = W.owner[lo];
-            const float4 en = __ldg(&P.cell_entries[W.cell[lo].x + (unsigned)(k - W.eoff[lo])]);
-            const float2 z = W.z[own];
-            const int t = f2i(en.z);
-            if (!(en.y < z.x || en.x > z.y) && t != W.excl[own]) {
-                float4 a, b, c;
-                if (t < P.smem_tris) {
-                    a = s_tris[3 * t]; b = s_tris[3 * t + 1]; c = s_tris[3 * t + 2];
-                } else {
-                    a = __ldg(&P.tris[3 * t]); b = __ldg(&P.tris[3 * t + 1]); c = __ldg(&P.tris[3 * t + 2]);
+            if (c < nk) W.eoff[c] = n_ent + inc - cnt;
+            n_ent += __shfl_sync(FULL, inc, 31);
+        }
+        __syncwarp();
+        for (int base = 0; base < n_ent; base += 32) {
+            const int k = base + lane;
+            if (k < n_ent) {
+                int lo = 0, hi = nk - 1;  // the entry's cell: the last kept cell whose offset is <= k
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (W.eoff[mid] <= k) lo = mid;
+                    else hi = mid - 1;
                 }
-                ++n_tri;
-                const float4 o = W.o[own], dd = W.d[own];
-                const float d = tri_distance(a, b, c, o.x, o.y, o.z, dd.x, dd.y, dd.z, retests);
-                if (d >= o.w && d <= dd.w) atomicMin(&W.best[own], pack_hit(__fadd_rn(d, 0.0f), (unsigned)t));
+                const int own = W.owner[lo];
+                const float4 en = __ldg(&P.cell_entries[W.cell[lo].x + (unsigned)(k - W.eoff[lo])]);
+                const float2 z = W.z[own];
+                const int t = f2i(en.z);
+                if (!(en.y < z.x || en.x > z.y) && t != W.excl[own]) {
+                    float4 a, b, c;
+                    if (t < P.smem_tris) {
+                        a = s_tris[3 * t]; b = s_tris[3 * t + 1]; c = s_tris[3 * t + 2];
+                    } else {
+                        a = __ldg(&P.tris[3 * t]); b = __ldg(&P.tris[3 * t + 1]); c = __ldg(&P.tris[3 * t + 2]);
+                    }
+                    ++n_tri;
+                    const float4 o = W.o[own], dd = W.d[own];
+                    const float d = tri_distance(a, b, c, o.x, o.y, o.z, dd.x, dd.y, dd.z, retests);
+                    if (d >= o.w && d <= dd.w) atomicMin(&W.best[own], pack_hit(__fadd_rn(d, 0.0f), (unsigned)t));
+                }
             }
         }
+        __syncwarp();
+        nk = 0;
     }
     __syncwarp();
     if (need && !fallback) {
@@ -241,11 +252,6 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
     const bool log_traj = kLog;
     const bool record_planes = P.mode == 1 || (P.flags & XMC_SCATTERING_MAP) != 0 || log_traj;
     unsigned xn = 0;  // crossings of the current photon (capacity + 1: the log overflowed)
-    // cooperative queries: a lane whose step needs the warp's query round waits (parked) until the
-    // round runs (query_batch lanes waiting, or every live lane); the step's draws and length are
-    // taken again when the round comes, exactly as the lane took them
-    bool parked = false;
-
     unsigned long long cbeg = 0, cend = 0;  // warp-uniform chunk of photon indices
     bool exhausted = false;                 // warp-uniform
     bool alive = false;
@@ -255,6 +261,19 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
     unsigned long long bias_gained = 0, bias_lost = 0;
     unsigned long long absorbed = 0, absorbed_out = 0, absorbed_tgt = 0;  // per-thread sums, flushed at the end
     unsigned budget_hit = 0;
+    // weight cut / roulette (mcml_kernel.cpp:121-124; planar GPU kernel.cu:214-222)
+    auto weight_cut = [&](float u) {
+        if (ph.w >= P.w_min) return;
+        if (!roulette) {
+            kill(S, ph, alive, L_N_CUT, L_CUT);
+        } else if (ph.w != 0u && u < P.chance) {
+            const WT nw = min(f2w<WT>(w2f(ph.w) * P.inv_chance), (WT)kWeightOne);
+            lat(&S.ledger[L_RGAINED], nw - ph.w);
+            ph.w = nw;
+        } else {
+            kill(S, ph, alive, L_N_ROULETTE, L_RKILLED);
+        }
+    };
 
     for (;;) {
         // ---- trajectory maps of the photons detected in the last iteration: the whole warp reads
@@ -331,8 +350,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
         // ---- no photons left to claim and few left in the warp: they go to the tail kernel ----
         if (exhausted && P.tail && __popc(living) <= kTailLanes) {
             if (alive) {
-                steps -= ph.iter;         // the tail kernel counts the whole walk
-                if (parked) ph.iter--;    // this step was drawn but not taken
+                steps -= ph.iter;  // the tail kernel counts the whole walk
                 unsigned xrow = 0;
                 if (log_traj) xrow = blockIdx.x * blockDim.x + threadIdx.x;
                 P.tail[atomicAdd(P.tail_count, 1u)] = TailPhoton::of(ph, xrow, xn);
@@ -340,13 +358,48 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
             break;
         }
 
-        // ---- one walk iteration (mcml_kernel.cpp:47-125) ----
+        // ---- free steps of every lane, until enough lanes wait for the general step below: a query, glass, a
+        // photon lost at the Area's faces, cut or at its step budget ----
+        const int batch = exhausted ? max(1, min(P.query_batch, __popc(living) / 4)) : P.query_batch;
+        bool wait = false;
+        unsigned waiting;
+        do {
+            if (alive && !wait) {
+                const uint4 r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter, 0u), P.key0,
+                                              P.key1);
+                const DevLayer& L = s_layer[ph.layer];
+                const float ox = ph.px, oy = ph.py, oz = ph.pz;
+                const float step = -__logf(u24(r.x)) * L.inv_mut;  // mcml_kernel.cpp:618-631
+                int idx;
+                WT dw;
+                wait = !free_step(P, L, step, area_kill, ph, idx, dw);
+                if (!wait) {
+                    steps++;
+                    if (idx >= 0) {
+                        if (dw && P.mode == 0) atomicAdd(&P.absorb[idx], (unsigned long long)dw);
+                        absorbed += dw;
+                    } else {
+                        absorbed_out += dw;
+                    }
+                    if ((P.target_mask >> ph.layer) & 1u) absorbed_tgt += dw;
+                    if (!(ph.pz > ph.gap_lo && ph.pz < ph.gap_hi))
+                        find_gap(s_zlo, s_zhi, P.n_zocc, ph.pz, ph.gap_lo, ph.gap_hi);
+                    if (record_planes) cross_planes(P, ox, oy, oz, ph.px, ph.py, ph.pz, ph.w + dw, ph.rdet,
+                                                    log_traj ? xlog_row(P, threadIdx.x) : nullptr, xn, n_cross);
+                    if constexpr (kBias) {  // the bias factor may take the weight below the cut
+                        biased_spin<1>(P, L, ph.layer, ph, bias_gained, bias_lost);
+                        weight_cut(u24(r.w));
+                    } else {
+                        hg_spin(L.hg_a, L.hg_b, L.hg_c, L.hg_d, L.hg_e, u24(r.y), u24(r.z), ph.dx, ph.dy, ph.dz);
+                    }
+                }
+            }
+            waiting = __ballot_sync(FULL, wait);
+        } while (__popc(waiting) < batch && waiting != (kBias ? __ballot_sync(FULL, alive) : living));
+
+        // ---- one walk iteration of the waiting lanes (mcml_kernel.cpp:47-125) ----
         // Up to the ray query no lane leaves the iteration, so that every lane reaches the query
-        // converged (the warp-cooperative query needs all 32); lanes with no photon or a photon that
-        // ends before it only skip the work.
-        bool act = alive && !parked;  // takes a new step this iteration
-        const bool fresh = act;
-        bool resumed = false;         // a waiting lane whose query round runs this iteration
+        // converged (the warp-cooperative query needs all 32).
         bool needq = false;
         float u_roulette = 0.0f;
         bool boundary = false;
@@ -356,11 +409,11 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
         float step = 0.0f;
         uint4 r = make_uint4(0u, 0u, 0u, 0u);
         const DevLayer* Lp = &s_layer[0];
-        if (act) {
+        if (wait) {
             if (ph.iter >= P.max_steps) {
                 budget_hit = 1;
                 kill(S, ph, alive, L_N_BUDGET, L_BUDGET);
-                act = false;
+                wait = false;
             } else {
                 r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter, 0u), P.key0, P.key1);
                 ph.iter++;
@@ -373,44 +426,26 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
                     u_roulette = u24(r.y);
                     if (hit.tri < 0) {
                         kill(S, ph, alive, L_N_GLASS, L_GLASS);
-                        act = false;
+                        wait = false;
                     } else {
                         step = hit.t;
                     }
                 } else {
-                    step = -__logf(u24(r.x)) * Lp->inv_mut;  // mcml_kernel.cpp:618-631
+                    step = -__logf(u24(r.x)) * Lp->inv_mut;
                     const float zend = fmaf(step + kStepExtend, ph.dz, ph.pz);
-                    if (fminf(ph.pz, zend) > ph.gap_lo && fmaxf(ph.pz, zend) < ph.gap_hi) {
-                        hit.tri = -1;  // the step stays inside a triangle-free z-gap: no surface to cross
-                        hit.t = step;
-                    } else {
-                        needq = true;
-                    }
+                    needq = !in_gap(ph, zend);
                 }
             }
         }
         if (P.grid_nx > 0 && P.coop_query) {
-            parked = parked || needq;
-            const unsigned pm = __ballot_sync(FULL, parked);
-            // with no photons left to claim the warp thins out: a long walk must not wait for as many others
-            // (planar stack with roulette, 1e6 photons: 62.9 -> 47.5 ms together with the hand-over)
-            const int batch = exhausted ? max(1, min(P.query_batch, __popc(living) / 4)) : P.query_batch;
-            if (pm && (__popc(pm) >= batch || pm == __ballot_sync(FULL, alive))) {
-                if (parked && !fresh) {
-                    Lp = &s_layer[ph.layer];
-                    r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter - 1u, 0u), P.key0,
-                                      P.key1);
-                    step = -__logf(u24(r.x)) * Lp->inv_mut;
-                }
+            if (__any_sync(FULL, needq)) {
                 bool fb = false;
-                warp_grid_query(P, *s_wq, s_big, s_tris, parked, ph.px, ph.py, ph.pz, ph.dx, ph.dy, ph.dz, ph.tmin,
+                warp_grid_query(P, *s_wq, s_big, s_tris, needq, ph.px, ph.py, ph.pz, ph.dx, ph.dy, ph.dz, ph.tmin,
                                 step + kStepExtend, ph.excl, hit, fb, retests, n_visit, n_tri);
-                if (parked && fb)
+                if (needq && fb)
                     hit = bvh_nearest(P.nodes, P.tris, P.n_nodes, s_nodes, P.smem_nodes, s_tris, P.smem_tris, ph.px,
                                       ph.py, ph.pz, ph.dx, ph.dy, ph.dz, ph.tmin, step + kStepExtend, ph.excl, retests,
                                       n_visit, n_tri);
-                resumed = parked;
-                parked = false;
             }
         } else if (needq) {
             if (!(P.grid_nx > 0 &&
@@ -421,7 +456,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
                                   ph.pz, ph.dx, ph.dy, ph.dz, ph.tmin, step + kStepExtend, ph.excl, retests, n_visit, n_tri);
             }
         }
-        if (!(act || resumed) || parked) continue;  // no photon, ended before its step, or waiting for its round
+        if (!wait) continue;
         const DevLayer& L = *Lp;
         if (!L.glass) {
             boundary = hit.tri >= 0;
@@ -487,22 +522,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
             ph.excl = -1;
             ph.tmin = 0.0f;
         }
-        // ---- weight cut / roulette (mcml_kernel.cpp:121-124; planar GPU kernel.cu:214-222) ----
-        if (ph.w < P.w_min) {
-            if (roulette) {
-                if (ph.w == 0u) {
-                    kill(S, ph, alive, L_N_ROULETTE, L_RKILLED);
-                } else if (u_roulette < P.chance) {
-                    const WT nw = min(f2w<WT>(w2f(ph.w) * P.inv_chance), (WT)kWeightOne);
-                    lat(&S.ledger[L_RGAINED], nw - ph.w);
-                    ph.w = nw;
-                } else {
-                    kill(S, ph, alive, L_N_ROULETTE, L_RKILLED);
-                }
-            } else {
-                kill(S, ph, alive, L_N_CUT, L_CUT);
-            }
-        }
+        weight_cut(u_roulette);
     }
 
     // ---- flush block-private tallies ----
@@ -681,11 +701,22 @@ extern "C" int xmc_debug_nearest(const InputInfo* in, int n_rays, const float* r
         return (flags & 2) ? XMC_ERR_DEVICE : XMC_ERR_INVALID_INPUT;
     }
     xmc::GridImage grid;
-    if (use_grid) xmc::build_xy_grid(g, &grid);
+    const bool use_clearance = (flags & 4) != 0;
+    if (use_grid || use_clearance) xmc::build_xy_grid(g, &grid);
+    xmc::KParams kp{};
+    std::vector<uint8_t> clear;
+    if (use_clearance) xmc::build_clearance(g, grid, &kp, &clear);
+    kp.clear = clear.data();
     for (int r = 0; r < n_rays; ++r) {
         const float* q = rays + 6 * (size_t)r;
         unsigned retests = 0, nv = 0, nt = 0;
         xmc::Hit h;
+        if (use_clearance) {
+            t_out[r] = xmc::clear_segment(kp, q[0], q[1], q[2], fmaf(q[3], tmax, q[0]), fmaf(q[4], tmax, q[1]),
+                                          fmaf(q[5], tmax, q[2])) ? 1.0f : 0.0f;
+            surf_out[r] = -1;
+            continue;
+        }
         if (!(use_grid && grid.nx > 0 && tmax < INFINITY &&
               xmc::grid_nearest(grid.cells.data(), grid.cell_z.data(), grid.entries.data(), grid.big.data(), (int)(grid.big.size() / 4), grid.x0,
                                 grid.y0, grid.icx, grid.icy, grid.nx, grid.ny, g.tris.data(), nullptr, 0, q[0], q[1], q[2],

@@ -5,19 +5,20 @@
 // Philox rounds, the logarithm, the angles and the optics one after the other); a run that has few photons
 // to begin with is all tail. Those photons come here (TailPhoton list, or the id dispenser itself for runs
 // of at most as many photons as the transport grid has threads) and a group of lanes walks each of them:
-//   * the random numbers do not depend on the path, so the lanes draw kTailGroup iterations at once, lane k
-//     the Philox block of iteration + k with its logarithm, Henyey-Greenstein angles and azimuth; what is
-//     left of a step is a short chain that every lane of the group runs on the same values;
-//   * a ray query tests one candidate triangle per lane;
-//   * a biased spin draws kTailGroup trials at once.
+//   * the random numbers do not depend on the path, so the lanes draw 16 iterations at once, each lane the
+//     Philox blocks of two of them with their logarithms, Henyey-Greenstein angles and azimuths;
+//   * a step that needs no ray query (free_step) is a short chain that every lane of the group runs on the
+//     same values and that a single branch leaves;
+//   * a ray query tests one candidate triangle per lane, and a biased spin draws 8 trials at once.
 // The arithmetic is the transport kernel's (walk.cuh, photon.cuh), so every tally is the same bit for bit.
 //
-// What bounds it: the dependent chain of a step (about 1,200 cycles with 16 warps per SM). Groups of 8
-// lanes beat whole warps (more photons per warp for the same chain; planar stack with roulette, 1e6 photons
-// 47.5 -> 43.8 ms) and groups of 4 or 16; 2 blocks per SM at 124 registers beat 3 at 80 (spills). A warp
-// hands its photons over when at most kTailLanes lanes hold one: 8 beat 4, 12 and 16 on most scenes.
-// B200, 1e6 photons, before -> with the tail kernel: planar stack with roulette 62.9 -> 43.8 ms, height
-// field 80.2 -> 57.1 ms, ellipsoid 66.3 -> 60.4 ms; 2e4 photons into the planar stack 5.6 -> 1.75 ms.
+// What bounds it: the latency of one step, 0.4 us of a lone photon (1.5 us in a warp of the transport kernel).
+// Groups of 8 lanes beat whole warps (more photons for the same chain; planar stack with roulette, 1e6
+// photons 47.5 -> 43.8 ms when this was the only change) and groups of 4 or 16; 2 blocks per SM at 128
+// registers beat 3 at 80 (spills). A warp hands its photons over when at most 8 lanes hold one: 4 and 16
+// were within 3 % and slower. Handing over every photon of 1,500 or 4,000 steps at once made it slower (29.8
+// and 31.5 ms against 28.6): here most photons are long walks. B200: 2e4 photons into the planar stack
+// 5.6 -> 1.75 ms, 901 under a glass cover 4.2 -> 0.9 ms; its share of larger runs is in transport.cu.
 #pragma once
 
 #include "walk.cuh"
@@ -28,13 +29,14 @@ namespace {
 
 constexpr int kTailThreads = 256;
 constexpr int kTailWarps = kTailThreads / 32;
-constexpr int kTailGroup = 8;  // lanes per photon (a power of two, at least kGridMaxCells)
-static_assert(kTailGroup >= kGridMaxCells, "one lane per cell of a query");
+constexpr int kTailGroup = 8;  // lanes per photon (a power of two)
 
-// The draws of a warp's groups, one iteration per lane: {step length, cos theta, sin theta, sin azimuth}, cos azimuth.
+constexpr int kTailDraws = 2;  // iterations that each lane draws at a time
+
+// The draws of a warp's groups: {step length, cos theta, sin theta, sin azimuth}, cos azimuth.
 struct TailDraws {
-    float4 a[32];
-    float cp[32];
+    float4 a[32 * kTailDraws];
+    float cp[32 * kTailDraws];
 };
 
 struct TailLayout {
@@ -59,7 +61,7 @@ __device__ __forceinline__ unsigned tail_group_mask() {
 
 // Nearest hit with tmin <= t <= tmax of one ray that all lanes of a group hold, over the big triangles and the entries
 // of the cells under the segment, one candidate per lane: the candidates and the choice of grid_nearest
-// (geom.cuh). False when the segment covers more than kGridMaxCells cells (the caller uses the BVH).
+// (geom.cuh). False when the segment covers more cells than the group has lanes (the caller uses the BVH).
 __device__ __forceinline__ bool tail_grid_query(const KParams& P, const float4* __restrict__ s_big,
                                                 const float4* __restrict__ s_tris, float ox, float oy, float oz, float dx,
                                                 float dy, float dz, float tmin, float tmax, int excl, Hit& hit,
@@ -76,7 +78,7 @@ __device__ __forceinline__ bool tail_grid_query(const KParams& P, const float4* 
     const int i0 = max(0, (int)floorf(fx0)), i1 = min(P.grid_nx - 1, (int)floorf(fx1));
     const int j0 = max(0, (int)floorf(fy0)), j1 = min(P.grid_ny - 1, (int)floorf(fy1));
     const int ww = i1 - i0 + 1, ncell = inside ? ww * (j1 - j0 + 1) : 0;
-    if (ncell > kGridMaxCells) return false;
+    if (ncell > G) return false;
     const float zl = fminf(oz, ez), zh = fmaxf(oz, ez);
     // this lane's cell: its entries that the segment's z-range can meet (cells_runs: per z-interval)
     uint2 cell = make_uint2(0u, 0u);
@@ -88,10 +90,6 @@ __device__ __forceinline__ bool tail_grid_query(const KParams& P, const float4* 
             cell.y = 0u;
         ++n_visit;
     }
-    const unsigned c0 = __shfl_sync(gm, cell.y, 0, G), c1 = c0 + __shfl_sync(gm, cell.y, 1, G);
-    const unsigned c2 = c1 + __shfl_sync(gm, cell.y, 2, G), total = c2 + __shfl_sync(gm, cell.y, 3, G);
-    const unsigned f0 = __shfl_sync(gm, cell.x, 0, G), f1 = __shfl_sync(gm, cell.x, 1, G) - c0;
-    const unsigned f2 = __shfl_sync(gm, cell.x, 2, G) - c1, f3 = __shfl_sync(gm, cell.x, 3, G) - c2;
     unsigned best_d = __float_as_uint(tmax), best_t = 0xffffffffu;
     auto candidate = [&](float4 a, float4 b, float4 c, int t) {
         ++n_tri;
@@ -107,12 +105,15 @@ __device__ __forceinline__ bool tail_grid_query(const KParams& P, const float4* 
         if (en.y < zl || en.x > zh || t == excl) continue;
         candidate(s_big[4 * k + 1], s_big[4 * k + 2], s_big[4 * k + 3], t);
     }
-    for (unsigned k = lane; k < total; k += G) {
-        const float4 en = __ldg(&P.cell_entries[k + (k < c0 ? f0 : k < c1 ? f1 : k < c2 ? f2 : f3)]);
-        const int t = f2i(en.z);
-        if (en.y < zl || en.x > zh || t == excl) continue;
-        if (t < P.smem_tris) candidate(s_tris[3 * t], s_tris[3 * t + 1], s_tris[3 * t + 2], t);
-        else candidate(__ldg(&P.tris[3 * t]), __ldg(&P.tris[3 * t + 1]), __ldg(&P.tris[3 * t + 2]), t);
+    for (int c = 0; c < ncell; ++c) {
+        const unsigned at = __shfl_sync(gm, cell.x, c, G), end = at + __shfl_sync(gm, cell.y, c, G);
+        for (unsigned k = at + lane; k < end; k += G) {
+            const float4 en = __ldg(&P.cell_entries[k]);
+            const int t = f2i(en.z);
+            if (en.y < zl || en.x > zh || t == excl) continue;
+            if (t < P.smem_tris) candidate(s_tris[3 * t], s_tris[3 * t + 1], s_tris[3 * t + 2], t);
+            else candidate(__ldg(&P.tris[3 * t]), __ldg(&P.tris[3 * t + 1]), __ldg(&P.tris[3 * t + 2]), t);
+        }
     }
     __syncwarp(gm);
     const unsigned d = __reduce_min_sync(gm, best_d);
@@ -128,8 +129,8 @@ template <bool kBias, bool kLog>
 __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const KParams P) {
     using WT = typename std::conditional<kBias, unsigned long long, uint32_t>::type;
     const unsigned n_listed = P.tail_direct ? 0u : *P.tail_count;
-    constexpr int G = kTailGroup;
-    if (!P.tail_direct && blockIdx.x * (kTailThreads / G) >= n_listed) return;  // nothing for this block
+    constexpr int G = kTailGroup, D = G * kTailDraws;
+    if (!P.tail_direct && blockIdx.x >= n_listed) return;  // nothing for this block
     extern __shared__ __align__(16) unsigned char smem[];
     const TailLayout lay = tail_layout(P);
     unsigned long long* s_ledger = reinterpret_cast<unsigned long long*>(smem);
@@ -140,6 +141,8 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
     DevDetector* s_det = reinterpret_cast<DevDetector*>(smem + lay.det);
     int8_t* s_next = reinterpret_cast<int8_t*>(smem + lay.next);
     TailDraws& W = reinterpret_cast<TailDraws*>(smem + lay.draws)[threadIdx.x >> 5];
+    float4* const draw = W.a + (threadIdx.x & 31) / G * D;
+    float* const draw_cp = W.cp + (threadIdx.x & 31) / G * D;
     __shared__ float s_zlo[kMaxZSlabs], s_zhi[kMaxZSlabs];
     __shared__ float4 s_big[4 * kMaxBigTriangles];
     for (int i = threadIdx.x; i < 4 * P.n_big; i += blockDim.x) s_big[i] = P.big[i];
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
     __syncthreads();
     const SmemTally S{s_ledger, s_dettal};
 
-    const int lane = threadIdx.x & (G - 1), at = threadIdx.x & 31 & ~(G - 1);  // of the group; its first lane
+    const int lane = threadIdx.x & (G - 1), first = threadIdx.x & 31 & ~(G - 1);  // of the group; its first lane
     const unsigned gm = tail_group_mask();
     const bool lead = lane == 0;  // the lane that adds the photon's tallies
     const bool area_kill = !(P.flags & XMC_NO_AREA_KILL);
@@ -166,6 +169,13 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
     unsigned long long bias_gained = 0, bias_lost = 0;
     unsigned long long absorbed = 0, absorbed_out = 0, absorbed_tgt = 0;
     unsigned budget_hit = 0;
+
+    // the first photons are dealt over the blocks, then over a block's warps, then over a warp's groups, so that
+    // few photons run on as many schedulers as there are; the rest come from the dispensers
+    const unsigned warps = gridDim.x * kTailWarps, n_groups = warps * (32 / G);
+    unsigned long long next = (unsigned long long)(first / G) * warps + (threadIdx.x / 32) * gridDim.x + blockIdx.x;
+    const unsigned long long n_next = P.tail_direct ? P.n_photons : (unsigned long long)n_listed;
+    bool dealt = true, done = false;
 
     Photon<WT> ph;
     unsigned xrow = 0, xn = 0;
@@ -177,21 +187,31 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
         }
         alive = false;
     };
-    int slot = G, layer = -1;  // next draw of the batch; the layer its step lengths and angles are for
-    uint4 r = make_uint4(0u, 0u, 0u, 0u);
+    int slot = D, layer = -1;  // next draw of the batch; the layer its step lengths and angles are for
+    uint4 r[kTailDraws];
+#pragma unroll
+    for (int j = 0; j < kTailDraws; ++j) r[j] = make_uint4(0u, 0u, 0u, 0u);
     for (;;) {
-        if (!alive) {
+        __syncwarp();  // lanes that branched off (tallies, groups at a surface) would each go on alone
+        if (!alive && !done) {
             // ---- this group's next photon ----
+            int cancelled = 0;
+            if (lead) {
+                if (P.tail_direct && P.cancel && *P.cancel) cancelled = 1;
+                if (!cancelled && !dealt)
+                    next = n_groups + (P.tail_direct ? atomicAdd(P.counter, 1ull) : (unsigned long long)atomicAdd(P.tail_next, 1u));
+            }
+            cancelled = __shfl_sync(gm, cancelled, 0, G);
+            next = __shfl_sync(gm, next, 0, G);
+            dealt = false;
+            done = cancelled || next >= n_next;
+            if (cancelled && lead) atomicOr(P.status, 2);
+        }
+        if (__all_sync(FULL, done)) break;
+        if (done) continue;
+        if (!alive) {
             if (P.tail_direct) {
-                unsigned long long idx = 0;
-                int cancelled = 0;
-                if (lead) {
-                    if (P.cancel && *P.cancel) cancelled = 1;
-                    idx = cancelled ? P.n_photons : atomicAdd(P.counter, 1ull);
-                    if (cancelled) atomicOr(P.status, 2);
-                }
-                idx = __shfl_sync(gm, idx, 0, G);
-                if (idx >= P.n_photons) break;
+                unsigned long long idx = next;
                 ph.rdet = -1;
                 if (P.mode == 1) {
                     const unsigned long long e = P.replay_list[idx];
@@ -203,11 +223,7 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
                 xn = 0;
                 if (lead) atomicAdd(&S.ledger[L_LAUNCHED], 1ull);
             } else {
-                unsigned e = 0;
-                if (lead) e = atomicAdd(P.tail_next, 1u);
-                e = __shfl_sync(gm, e, 0, G);
-                if (e >= n_listed) break;
-                const TailPhoton& T = P.tail[e];
+                const TailPhoton& T = P.tail[next];
                 ph.px = T.px; ph.py = T.py; ph.pz = T.pz;
                 ph.dx = T.dx; ph.dy = T.dy; ph.dz = T.dz;
                 ph.time = T.time; ph.trange = T.trange; ph.orange = T.orange; ph.tmin = T.tmin;
@@ -219,33 +235,71 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
             find_gap(s_zlo, s_zhi, P.n_zocc, ph.pz, ph.gap_lo, ph.gap_hi);
             if (kLog) ph.rdet = -1;
             alive = true;
-            slot = G;
+            slot = D;
         }
         unsigned* const xl = kLog ? P.xlog + (size_t)xrow * P.xlog_cap : nullptr;
+        if (slot == D || layer != ph.layer) {
+            if (slot == D) {
+#pragma unroll
+                for (int j = 0; j < kTailDraws; ++j)
+                    r[j] = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter + G * j + lane, 0u), P.key0,
+                                         P.key1);
+                slot = 0;
+            }
+            layer = ph.layer;
+            const DevLayer& L = s_layer[layer];
+            __syncwarp(gm);  // every lane has read the previous draws
+#pragma unroll
+            for (int j = 0; j < kTailDraws; ++j) {
+                float4 a;
+                float cp = 0.0f;
+                a.x = -__logf(u24(r[j].x)) * L.inv_mut;
+                if (!kBias) hg_angles(L.hg_a, L.hg_b, L.hg_c, L.hg_d, L.hg_e, u24(r[j].y), u24(r[j].z), a.y, a.z, a.w, cp);
+                draw[G * j + lane] = a;
+                draw_cp[G * j + lane] = cp;
+            }
+            __syncwarp(gm);
+        }
+        // ---- free steps: one short chain each, left by a single branch ----
+        if (!kBias) {
+            const DevLayer& L = s_layer[layer];
+            const bool target = (P.target_mask >> layer) & 1u;
+            while (slot < D) {
+                const float4 A = draw[slot];
+                const float ox = ph.px, oy = ph.py, oz = ph.pz;
+                int idx;
+                WT dw;
+                if (!free_step(P, L, A.x, area_kill, ph, idx, dw)) break;
+                if (idx >= 0) {
+                    if (lead && dw && P.mode == 0) atomicAdd(&P.absorb[idx], (unsigned long long)dw);
+                    absorbed += dw;
+                } else {
+                    absorbed_out += dw;
+                }
+                if (target) absorbed_tgt += dw;
+                if (!(ph.pz > ph.gap_lo && ph.pz < ph.gap_hi))
+                    find_gap(s_zlo, s_zhi, P.n_zocc, ph.pz, ph.gap_lo, ph.gap_hi);
+                if (record_planes) {
+                    if (lead) cross_planes(P, ox, oy, oz, ph.px, ph.py, ph.pz, ph.w + dw, ph.rdet, xl, xn, n_cross);
+                    __syncwarp(gm);
+                }
+                hg_rotate(A.y, A.z, A.w, draw_cp[slot], ph.dx, ph.dy, ph.dz);
+                ++slot;
+            }
+            if (slot == D) continue;
+        }
         // ---- one walk iteration (the transport kernel's) ----
         if (ph.iter >= P.max_steps) {
             budget_hit = 1;
             die(L_N_BUDGET, L_BUDGET);
             continue;
         }
-        if (slot == G || layer != ph.layer) {
-            if (slot == G) {
-                r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter + lane, 0u), P.key0, P.key1);
-                slot = 0;
-            }
-            layer = ph.layer;
-            const DevLayer& L = s_layer[layer];
-            float4 a;
-            float cp = 0.0f;
-            a.x = -__logf(u24(r.x)) * L.inv_mut;
-            if (!kBias) hg_angles(L.hg_a, L.hg_b, L.hg_c, L.hg_d, L.hg_e, u24(r.y), u24(r.z), a.y, a.z, a.w, cp);
-            __syncwarp(gm);  // every lane has read the previous draws
-            W.a[at + lane] = a;
-            W.cp[at + lane] = cp;
-            __syncwarp(gm);
-        }
         const int k = slot++;
-        const float4 A = W.a[at + k];
+        const float4 A = draw[k];
+        uint4 rk = r[0];
+#pragma unroll
+        for (int j = 1; j < kTailDraws; ++j)
+            if (k / G == j) rk = r[j];
         ph.iter++;
         const DevLayer& L = s_layer[layer];
         Hit hit;
@@ -263,7 +317,7 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
             boundary = true;
         } else {
             const float zend = fmaf(step + kStepExtend, ph.dz, ph.pz);
-            if (!(fminf(ph.pz, zend) > ph.gap_lo && fmaxf(ph.pz, zend) < ph.gap_hi)) {
+            if (!in_gap(ph, zend)) {
                 if (!(P.grid_nx > 0 && tail_grid_query(P, s_big, s_tris, ph.px, ph.py, ph.pz, ph.dx, ph.dy, ph.dz, ph.tmin,
                                                        step + kStepExtend, ph.excl, hit, retests, n_visit, n_tri)))
                     hit = bvh_nearest(P.nodes, P.tris, P.n_nodes, s_nodes, P.smem_nodes, s_tris, P.smem_tris, ph.px, ph.py,
@@ -289,7 +343,7 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
             continue;
         }
         if (boundary) {
-            const uint32_t uf = __shfl_sync(gm, L.glass ? r.x : r.y, k, G);
+            const uint32_t uf = __shfl_sync(gm, L.glass ? rk.x : rk.y, k, G);
             const int crossed = cross_boundary(P, s_layer, s_tris, s_next, L, hit.tri, u24(uf), ph);
             if (crossed == kCrossInvalid) {
                 die(L_N_INVALID, L_INVALID);
@@ -330,14 +384,14 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
             if ((P.target_mask >> layer) & 1u) absorbed_tgt += dw;
             // ---- spin (mcml_kernel.cpp:442-495) ----
             if constexpr (kBias) biased_spin<G>(P, L, layer, ph, bias_gained, bias_lost);
-            else hg_rotate(A.y, A.z, A.w, W.cp[at + k], ph.dx, ph.dy, ph.dz);
+            else hg_rotate(A.y, A.z, A.w, draw_cp[k], ph.dx, ph.dy, ph.dz);
             ph.excl = -1;
             ph.tmin = 0.0f;
         }
         // ---- weight cut / roulette ----
         if (ph.w < P.w_min) {
             if (roulette) {
-                const float u = u24(__shfl_sync(gm, L.glass ? r.y : boundary ? r.z : r.w, k, G));
+                const float u = u24(__shfl_sync(gm, L.glass ? rk.y : boundary ? rk.z : rk.w, k, G));
                 if (ph.w != 0u && u < P.chance) {
                     const WT nw = min(f2w<WT>(w2f(ph.w) * P.inv_chance), (WT)kWeightOne);
                     if (lead) lat(&S.ledger[L_RGAINED], nw - ph.w);

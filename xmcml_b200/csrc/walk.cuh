@@ -305,6 +305,40 @@ __device__ __forceinline__ void biased_spin(const KParams& P, const DevLayer& L,
     ph.dx = nx; ph.dy = ny; ph.dz = nz;
 }
 
+// Whether a step that passes over the z-range [pz, zend] stays in the photon's triangle-free z-gap.
+template <class Ph>
+__device__ __forceinline__ bool in_gap(const Ph& ph, float zend) {
+    return fminf(ph.pz, zend) > ph.gap_lo && fmaxf(ph.pz, zend) < ph.gap_hi;
+}
+
+// An interaction step that needs no ray query (it stays inside the photon's triangle-free z-gap, or clear of
+// every triangle), does not end outside Area where that kills, and leaves the weight at or above the cut: moves the photon and drops `dw`
+// into voxel `idx` (-1: outside Area). False, with nothing changed, for any other step.
+template <class Ph, typename WT>
+__device__ __forceinline__ bool free_step(const KParams& P, const DevLayer& L, float step, bool area_kill, Ph& ph, int& idx,
+                                          WT& dw) {
+    const float zend = fmaf(step + kStepExtend, ph.dz, ph.pz);
+    const float nx = fmaf(step, ph.dx, ph.px), ny = fmaf(step, ph.dy, ph.py), nz = fmaf(step, ph.dz, ph.pz);
+    idx = area_index(P, nx, ny, nz, 0.0f);
+    dw = f2w<WT>(w2f(ph.w) * L.absorb);
+    dw = min(dw, ph.w);
+    if ((idx < 0 && area_kill) || ph.w - dw < P.w_min || ph.iter >= P.max_steps || L.glass) return false;
+    if (!in_gap(ph, zend) && !clear_segment(P, ph.px, ph.py, ph.pz, fmaf(step + kStepExtend, ph.dx, ph.px),
+                                            fmaf(step + kStepExtend, ph.dy, ph.py), zend))
+        return false;
+    ph.px = nx;
+    ph.py = ny;
+    ph.pz = nz;
+    ph.time = fmaf(step, L.n, ph.time);
+    if ((P.target_mask >> ph.layer) & 1u) ph.trange += step;
+    else ph.orange += step;
+    ph.w -= dw;
+    ph.excl = -1;
+    ph.tmin = 0.0f;
+    ph.iter++;
+    return true;
+}
+
 // CrossBoundary (mcml_kernel.cpp:229-284) at triangle `tri`, hit from layer L: Fresnel test against
 // `u_fresnel`, then refraction or reflection. Returns kCrossInvalid when the surface leads nowhere from
 // this layer, kCrossLeft when the photon leaves the tissue (its direction unchanged, for the detectors),
