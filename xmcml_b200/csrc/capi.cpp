@@ -213,6 +213,8 @@ int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img
     kp.nx = A.partitionNumber.x; kp.ny = A.partitionNumber.y; kp.nz = A.partitionNumber.z;
     kp.byte_sentinel = (A.partitionNumber.x >= 256 && A.partitionNumber.y >= 256 && A.partitionNumber.z >= 256 &&
                         !(opt.flags & XMC_LARGE_GRID)) ? 1 : 0;
+    kp.voxel_bias = 0u - 0x4B000000u * (uint32_t)(kp.ny * kp.nz + kp.nz + 1);
+    kp.voxel_sentinel = kp.byte_sentinel ? (uint32_t)((255 * kp.ny + 255) * kp.nz + 255) : 0xffffffffu;
     img->grid_size = A.partitionNumber.x * A.partitionNumber.y * A.partitionNumber.z;
     kp.grid = img->grid_size;
     kp.plane_dz = (float)(A.length.z / A.partitionNumber.z);
@@ -281,7 +283,7 @@ int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img
     kp.chance = (float)opt.roulette_chance;
     kp.inv_chance = (float)(1.0 / opt.roulette_chance);
     kp.flags = opt.flags;
-    kp.max_steps = opt.max_steps_per_photon;
+    kp.max_steps = (uint32_t)std::min<unsigned long long>(opt.max_steps_per_photon, 0xffffffffull);
     kp.chunk = opt.photons_per_chunk;
 
     // ---- shared-memory staging plan ----
@@ -600,8 +602,7 @@ static int run(Context* c, uint64_t seed, uint64_t first, uint64_t n, OutputInfo
     xmc::DeviceGuard device_guard;  // the caller's current device is restored on return
     XMC_CUDA(cudaSetDevice(c->device));
     KParams& kp = c->kp;
-    kp.key0 = (uint32_t)seed;
-    kp.key1 = (uint32_t)(seed >> 32);
+    kp.keys = philox_round_keys((uint32_t)seed, (uint32_t)(seed >> 32));
     kp.first_id = first;
     kp.n_photons = n;
     const size_t absorb_b = sizeof(unsigned long long) * (size_t)c->grid_size;

@@ -141,8 +141,7 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     kp.det = d_detectors;
     kp.tbin = d_time_bins;
     kp.ledger = d_ledger;
-    kp.key0 = (uint32_t)seed;
-    kp.key1 = (uint32_t)(seed >> 32);
+    kp.keys = philox_round_keys((uint32_t)seed, (uint32_t)(seed >> 32));
     kp.first_id = first_photon_id;
     kp.n_photons = n_photons;
 

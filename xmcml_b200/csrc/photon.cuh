@@ -3,6 +3,7 @@
 // near-critical-angle Fresnel branch, which is FP64.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 
 namespace xmc {
@@ -26,6 +27,31 @@ __host__ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint32_t k0, ui
     }
     return c;
 }
+
+// The same with the key schedule worked out beforehand (philox_round_keys): the round keys come from the
+// kernel's parameters as operands of the rounds' XORs instead of two additions per round.
+struct PhiloxKeys {
+    uint32_t k0[10], k1[10];
+};
+inline PhiloxKeys philox_round_keys(uint32_t k0, uint32_t k1) {
+    PhiloxKeys k;
+    for (int r = 0; r < 10; ++r) {
+        k.k0[r] = k0 + (uint32_t)r * 0x9E3779B9u;
+        k.k1[r] = k1 + (uint32_t)r * 0xBB67AE85u;
+    }
+    return k;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ uint4 philox4x32_10(uint4 c, const PhiloxKeys& k) {
+#pragma unroll
+    for (int r = 0; r < 10; ++r) {
+        const uint32_t lo0 = 0xD2511F53u * c.x, hi0 = __umulhi(0xD2511F53u, c.x);
+        const uint32_t lo1 = 0xCD9E8D57u * c.z, hi1 = __umulhi(0xCD9E8D57u, c.z);
+        c = make_uint4(hi1 ^ c.y ^ k.k0[r], lo1, hi0 ^ c.w ^ k.k1[r], lo0);
+    }
+    return c;
+}
+#endif
 
 // 24-bit uniform in (0,1), exactly the value the FP64 oracle uses.
 __host__ __device__ __forceinline__ float u24(uint32_t x) { return fmaf((float)(x >> 8), 0x1p-24f, 0x1p-25f); }
@@ -74,12 +100,8 @@ __device__ __forceinline__ float radius_xy(float x, float y) { return sqrtf(__fm
 // hg_e == 0) and sin(theta); sine and cosine of the azimuth 2 pi u2. It does not depend on the direction.
 __device__ __forceinline__ void hg_angles(float hg_a, float hg_b, float hg_c, float hg_d, float hg_e, float u1, float u2,
                                           float& cost, float& sint, float& sp, float& cp) {
-    if (hg_e != 0.0f) {
-        const float t = hg_a / (hg_d + hg_e * u1);
-        cost = (hg_b - t * t) * hg_c;
-    } else {
-        cost = 2.0f * u1 - 1.0f;
-    }
+    const float t = hg_a / (hg_d + hg_e * u1);
+    cost = hg_e != 0.0f ? (hg_b - t * t) * hg_c : 2.0f * u1 - 1.0f;
     cost = fminf(1.0f, fmaxf(-1.0f, cost));
     sint = sqrtf(fmaxf(0.0f, 1.0f - cost * cost));
     float a = u2;
@@ -91,23 +113,20 @@ __device__ __forceinline__ void hg_angles(float hg_a, float hg_b, float hg_c, fl
 // near-vertical special case.
 __device__ __forceinline__ void hg_rotate(float cost, float sint, float sp, float cp, float& dx, float& dy, float& dz) {
     const float ux = dx, uy = dy, uz = dz;
-    const float rho2 = ux * ux + uy * uy;
-    float nx, ny, nz;
-    if (rho2 > 1e-12f) {
-        const float irho = rsqrtf(rho2);
-        const float rho = rho2 * irho;
-        nx = sint * (ux * uz * cp - uy * sp) * irho + ux * cost;
-        ny = sint * (uy * uz * cp + ux * sp) * irho + uy * cost;
-        nz = -sint * cp * rho + uz * cost;
-    } else {
-        nx = sint * cp;
-        ny = sint * sp;
-        nz = uz >= 0.0f ? cost : -cost;
-    }
-    const float on = rsqrtf(nx * nx + ny * ny + nz * nz);
-    dx = nx * on;
-    dy = ny * on;
-    dz = nz * on;
+    // the rounding of every sum is written out (see fresnel_reflectance), and both cases are computed: a branch
+    // for the rare one would end the straight line that the compiler schedules the random numbers into
+    const float rho2 = __fmaf_rn(uy, uy, __fmul_rn(ux, ux));
+    const float irho = rsqrtf(rho2);
+    const float rho = __fmul_rn(rho2, irho);
+    const float ax = __fmaf_rn(__fmul_rn(ux, uz), cp, -__fmul_rn(uy, sp)), ay = __fmaf_rn(ux, sp, __fmul_rn(__fmul_rn(uy, uz), cp));
+    const bool slanted = rho2 > 1e-12f;
+    const float nx = slanted ? __fmaf_rn(ux, cost, __fmul_rn(__fmul_rn(sint, ax), irho)) : __fmul_rn(sint, cp);
+    const float ny = slanted ? __fmaf_rn(uy, cost, __fmul_rn(__fmul_rn(sint, ay), irho)) : __fmul_rn(sint, sp);
+    const float nz = slanted ? __fmaf_rn(uz, cost, __fmul_rn(__fmul_rn(-sint, cp), rho)) : uz >= 0.0f ? cost : -cost;
+    const float on = rsqrtf(__fmaf_rn(nz, nz, __fmaf_rn(nx, nx, __fmul_rn(ny, ny))));
+    dx = __fmul_rn(nx, on);
+    dy = __fmul_rn(ny, on);
+    dz = __fmul_rn(nz, on);
 }
 
 __device__ __forceinline__ void hg_spin(float hg_a, float hg_b, float hg_c, float hg_d, float hg_e, float u1, float u2,

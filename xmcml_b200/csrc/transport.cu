@@ -365,8 +365,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
         unsigned waiting;
         do {
             if (alive && !wait) {
-                const uint4 r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter, 0u), P.key0,
-                                              P.key1);
+                const uint4 r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter, 0u), P.keys);
                 const DevLayer& L = s_layer[ph.layer];
                 const float ox = ph.px, oy = ph.py, oz = ph.pz;
                 const float step = -__logf(u24(r.x)) * L.inv_mut;  // mcml_kernel.cpp:618-631
@@ -415,7 +414,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
                 kill(S, ph, alive, L_N_BUDGET, L_BUDGET);
                 wait = false;
             } else {
-                r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter, 0u), P.key0, P.key1);
+                r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter, 0u), P.keys);
                 ph.iter++;
                 steps++;
                 Lp = &s_layer[ph.layer];

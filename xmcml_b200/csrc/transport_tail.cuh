@@ -242,8 +242,7 @@ __global__ void __launch_bounds__(kTailThreads, 2) transport_tail_kernel(const K
             if (slot == D) {
 #pragma unroll
                 for (int j = 0; j < kTailDraws; ++j)
-                    r[j] = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter + G * j + lane, 0u), P.key0,
-                                         P.key1);
+                    r[j] = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter + G * j + lane, 0u), P.keys);
                 slot = 0;
             }
             layer = ph.layer;

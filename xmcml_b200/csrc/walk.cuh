@@ -222,7 +222,7 @@ __device__ __forceinline__ void launch_photon(const KParams& P, Ph& ph, unsigned
     ph.py = P.sy;
     ph.pz = P.sz;
     if (P.beam_radius > 0.0f) {
-        const uint4 r = philox4x32_10(make_uint4((uint32_t)pid, (uint32_t)(pid >> 32), 0u, 1u), P.key0, P.key1);
+        const uint4 r = philox4x32_10(make_uint4((uint32_t)pid, (uint32_t)(pid >> 32), 0u, 1u), P.keys);
         const float rad = P.beam_radius * sqrtf(u24(r.x));
         float a = u24(r.y);
         a = a > 0.5f ? a - 1.0f : a;
@@ -273,7 +273,7 @@ __device__ __forceinline__ void biased_spin(const KParams& P, const DevLayer& L,
     float nx = ph.dx, ny = ph.dy, nz = ph.dz, p = 1.0f;
     for (uint32_t k = threadIdx.x & (kLanes - 1); k < kBiasMaxTrials; k += kLanes) {
         const uint4 r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter - 1u, 2u + k),
-                                      P.key0, P.key1);
+                                      P.keys);
         nx = ph.dx; ny = ph.dy; nz = ph.dz;
         hg_spin(L.hg_a, L.hg_b, L.hg_c, L.hg_d, L.hg_e, u24(r.x), u24(r.y), nx, ny, nz);
         p = powf(fmaf(0.45f, 1.0f + (nx * vx + ny * vy + nz * vz), 0.1f), P.bias_eps);
@@ -308,7 +308,7 @@ __device__ __forceinline__ void biased_spin(const KParams& P, const DevLayer& L,
 // Whether a step that passes over the z-range [pz, zend] stays in the photon's triangle-free z-gap.
 template <class Ph>
 __device__ __forceinline__ bool in_gap(const Ph& ph, float zend) {
-    return fminf(ph.pz, zend) > ph.gap_lo && fmaxf(ph.pz, zend) < ph.gap_hi;
+    return (fminf(ph.pz, zend) > ph.gap_lo) & (fmaxf(ph.pz, zend) < ph.gap_hi);
 }
 
 // An interaction step that needs no ray query (it stays inside the photon's triangle-free z-gap, or clear of
@@ -319,10 +319,16 @@ __device__ __forceinline__ bool free_step(const KParams& P, const DevLayer& L, f
                                           WT& dw) {
     const float zend = fmaf(step + kStepExtend, ph.dz, ph.pz);
     const float nx = fmaf(step, ph.dx, ph.px), ny = fmaf(step, ph.dy, ph.py), nz = fmaf(step, ph.dz, ph.pz);
-    idx = area_index(P, nx, ny, nz, 0.0f);
+    // area_index with tol 0 and no branch: inside Area the coordinates are in [0, 4096), so that adding 2^23
+    // towards zero leaves their integer parts in the float's low bits, and the bits above cancel in voxel_bias
+    const float fx = (nx - P.ax) * P.asx, fy = (ny - P.ay) * P.asy, fz = (nz - P.az) * P.asz;
+    const bool inside = (fx >= 0.0f) & (fy >= 0.0f) & (fz >= 0.0f) & (fx < (float)P.nx) & (fy < (float)P.ny) & (fz < (float)P.nz);
+    const uint32_t bx = __float_as_uint(__fadd_rz(fx, 8388608.0f)), by = __float_as_uint(__fadd_rz(fy, 8388608.0f));
+    const uint32_t voxel = (bx * (uint32_t)P.ny + by) * (uint32_t)P.nz + __float_as_uint(__fadd_rz(fz, 8388608.0f)) + P.voxel_bias;
+    idx = inside & (voxel != P.voxel_sentinel) ? (int)voxel : -1;
     dw = f2w<WT>(w2f(ph.w) * L.absorb);
     dw = min(dw, ph.w);
-    if ((idx < 0 && area_kill) || ph.w - dw < P.w_min || ph.iter >= P.max_steps || L.glass) return false;
+    if ((idx < 0) & area_kill | (ph.w - dw < P.w_min) | (ph.iter >= P.max_steps) | (L.glass != 0)) return false;
     if (!in_gap(ph, zend) && !clear_segment(P, ph.px, ph.py, ph.pz, fmaf(step + kStepExtend, ph.dx, ph.px),
                                             fmaf(step + kStepExtend, ph.dy, ph.py), zend))
         return false;

@@ -8,6 +8,8 @@
 
 #include <cuda_runtime.h>
 
+#include "photon.cuh"
+
 // CUDA's vector_types.h also defines double3 and int3; inside this library the reference's
 // vertex and index types are named xmc_ref_double3 / xmc_ref_int3 (same layout, same union tags).
 #define double3 xmc_ref_double3
@@ -191,6 +193,8 @@ struct KParams {
     float ax, ay, az;         // corner
     float asx, asy, asz;      // partitions / length
     int nx, ny, nz;
+    uint32_t voxel_bias;      // free_step: what the voxel indices' float bits add to the index
+    uint32_t voxel_sentinel;  // index of that voxel, 0xffffffff without one
     int byte_sentinel;        // voxel (255,255,255) counts as outside (reference byte index semantics)
     // detectors and time bins
     const DevDetector* dets;
@@ -206,8 +210,9 @@ struct KParams {
     uint32_t w_min;           // minWeight (fixed point)
     float chance, inv_chance; // roulette
     uint32_t flags;
-    uint32_t key0, key1;      // Philox key (seed)
-    unsigned long long first_id, n_photons, max_steps;
+    PhiloxKeys keys;          // Philox round keys of the seed
+    unsigned long long first_id, n_photons;
+    uint32_t max_steps;       // per photon
     int chunk;
     // z-plane crossing tallies (UpdatePhotonTrajectory): planes at voxel centres
     float plane_dz;           // Area length.z / partitions.z
