@@ -69,14 +69,32 @@ __device__ __forceinline__ void warp_rows_f32(float* sw, const float (&v)[32], f
     }
     __syncwarp();
 }
-__device__ __forceinline__ void warp_rows_bf16(float* sw, const float (&v)[32], bf16* dst, size_t ld, int row0, int col0,
-                                               int lane) {
+// The lane's 32 columns of its own row: four 16-byte stores, which fill whole 32-byte sectors. (Through the
+// shared-memory tile, 32 stores of 64 bytes per warp, the epilogue took three times the instructions.)
+__device__ __forceinline__ void lane_row_bf16(const float (&v)[32], bf16* dst) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) sw[lane * 33 + j] = v[j];
-    __syncwarp();
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k) dst[(size_t)(row0 + k) * ld + col0 + lane] = __float2bfloat16_rn(sw[k * 33 + lane]);
-    __syncwarp();
+    for (int j = 0; j < 4; ++j) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        reinterpret_cast<uint4*>(dst)[j] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// r[] plus the bias of its 32 columns (the same for every lane).
+__device__ __forceinline__ void add_bias(const uint32_t (&r)[32], const float* __restrict__ bias, float (&v)[32]) {
+    const float4* b4 = reinterpret_cast<const float4*>(bias);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const float4 b = __ldg(&b4[q]);
+        v[4 * q] = f32(r[4 * q]) + b.x;
+        v[4 * q + 1] = f32(r[4 * q + 1]) + b.y;
+        v[4 * q + 2] = f32(r[4 * q + 2]) + b.z;
+        v[4 * q + 3] = f32(r[4 * q + 3]) + b.w;
+    }
 }
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + __expf(-z)); }
@@ -110,12 +128,11 @@ struct EpiHidden {
     int ldt;
     __device__ void apply(int row, int col0, const uint32_t (&r)[32], int lane, float* sw) const {
         float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = f32(r[j]) + __ldg(&bias[col0 + j]);
-        if (z) warp_rows_bf16(sw, v, z, (size_t)lda, row - lane, col0, lane);
+        add_bias(r, bias + col0, v);
+        if (z) lane_row_bf16(v, z + (size_t)row * lda + col0);
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = silu(v[j]);
-        warp_rows_bf16(sw, v, a, (size_t)lda, row - lane, col0, lane);
+        lane_row_bf16(v, a + (size_t)row * lda + col0);
         if (at) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) at[(size_t)(col0 + j) * ldt + row] = __float2bfloat16_rn(v[j]);
@@ -125,14 +142,16 @@ struct EpiHidden {
 
 // Output layer: Y = acc + b for the first n_out columns. Training (t != nullptr): the gradient of
 // the (optionally per-output weighted) mean squared error dY = scale w (Y - T) (0 in the padding
-// columns), row-major and transposed, and the sum of w (Y - T)^2 added to loss[*step].
+// columns), row-major and transposed, and the sum of w (Y - T)^2 added to loss[*step + step_add]. The targets
+// of row i are row src[i] of t (row i without src): they are read where the data set holds them.
 struct EpiOut {
     const float* bias;
     float* y;  // nullable, [rows x ldy]
     int ldy;
     int n_out;
-    const float* t;  // nullable, [rows x ldtg]
+    const float* t;  // nullable, [. x ldtg]
     int ldtg;
+    const int* src;  // nullable
     bf16* dy;
     int lddy;
     bf16* dyt;
@@ -141,28 +160,52 @@ struct EpiOut {
     const float* colw;  // nullable: per-output weight of the squared error
     float* loss;
     const int* step;
+    int step_add;
     __device__ void apply(int row, int col0, const uint32_t (&r)[32], int lane, float* sw) const {
         float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = f32(r[j]) + __ldg(&bias[col0 + j]);
+        add_bias(r, bias + col0, v);
         if (y && col0 < n_out) warp_rows_f32(sw, v, y, (size_t)ldy, row - lane, col0, n_out, lane);
         if (t) {
+            const int own = src ? __ldg(&src[row]) : row;
+            if ((ldtg & 3) == 0 && col0 + 32 <= n_out && (reinterpret_cast<uintptr_t>(t) & 15) == 0) {
+                // the lane's own row, eight 16-byte loads in flight (33 -> 17 us of the layer at 4,096 rows x 1,000)
+                const float4* tp = reinterpret_cast<const float4*>(t + (size_t)own * ldtg + col0);
+                float4 q[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) q[j] = __ldg(&tp[j]);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    sw[lane * 33 + 4 * j] = q[j].x;
+                    sw[lane * 33 + 4 * j + 1] = q[j].y;
+                    sw[lane * 33 + 4 * j + 2] = q[j].z;
+                    sw[lane * 33 + 4 * j + 3] = q[j].w;
+                }
+            } else {
+                // rows of any alignment, through the warp's tile along their columns
+                const bool col = col0 + lane < n_out;
+#pragma unroll 8
+                for (int k = 0; k < 32; ++k) {
+                    const float* tp = t + (size_t)__shfl_sync(0xffffffffu, own, k) * ldtg + col0 + lane;
+                    sw[k * 33 + lane] = col ? __ldg(tp) : 0.0f;
+                }
+            }
+            __syncwarp();
             float se = 0.0f;
-            const float* tp = t + (size_t)row * ldtg;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 const int c = col0 + j;
-                const float d = c < n_out ? v[j] - __ldg(&tp[c]) : 0.0f;
+                const float d = c < n_out ? v[j] - sw[lane * 33 + j] : 0.0f;
                 const float wd = (colw && c < n_out) ? d * __ldg(&colw[c]) : d;
                 se = fmaf(wd, d, se);
                 v[j] = wd * scale;
             }
-            warp_rows_bf16(sw, v, dy, (size_t)lddy, row - lane, col0, lane);
+            __syncwarp();
+            lane_row_bf16(v, dy + (size_t)row * lddy + col0);
 #pragma unroll
             for (int j = 0; j < 32; ++j) dyt[(size_t)(col0 + j) * lddyt + row] = __float2bfloat16_rn(v[j]);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
-            if (lane == 0) atomicAdd(loss + *step, se);
+            if (lane == 0) atomicAdd(loss + *step + step_add, se);
         }
     }
 };
@@ -179,7 +222,7 @@ struct EpiBwd {
         load_bf16x32(z + (size_t)row * ldz + col0, zv);
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = f32(r[j]) * dsilu(zv[j]);
-        warp_rows_bf16(sw, v, dz, (size_t)ldz, row - lane, col0, lane);
+        lane_row_bf16(v, dz + (size_t)row * ldz + col0);
 #pragma unroll
         for (int j = 0; j < 32; ++j) dzt[(size_t)(col0 + j) * ldt + row] = __float2bfloat16_rn(v[j]);
     }
@@ -198,44 +241,58 @@ __global__ void pack_inputs_kernel(const float* __restrict__ x, int rows, int n_
     if (xt) xt[(size_t)c * ldt + r] = v;
 }
 
-// Minibatch of `rows` rows drawn with replacement from the device data set (Philox keyed by seed,
-// counter (step, row)): inputs (bf16, padded, and transposed) and FP32 targets.
-__global__ void gather_kernel(const bf16* __restrict__ ds_x, const float* __restrict__ ds_t, int ds_rows, int n_out,
-                              int rows, uint32_t k0, uint32_t k1, const int* __restrict__ step, bf16* __restrict__ xb,
-                              bf16* __restrict__ xt, float* __restrict__ tb) {
-    const int r = blockIdx.x;
-    __shared__ int src;
-    if (threadIdx.x == 0) {
-        const uint4 u = philox4x32_10(make_uint4((uint32_t)r, (uint32_t)*step, 0x6d6c70u, 0u), k0, k1);
-        src = (int)(((unsigned long long)u.x * (unsigned long long)ds_rows) >> 32);
+// Minibatch of `rows` rows drawn with replacement from the device data set (Philox keyed by seed, counter
+// (step, row)) for step *step + 1: inputs (bf16, padded, and transposed) and the rows' places in the data
+// set, where the output layer reads their targets. 32 rows per block, a warp per four.
+__global__ void gather_kernel(const bf16* __restrict__ ds_x, int ds_rows, int rows, uint32_t k0, uint32_t k1,
+                              const int* __restrict__ step, float* __restrict__ loss, bf16* __restrict__ xb,
+                              bf16* __restrict__ xt, int* __restrict__ src, const float* __restrict__ ds_t, int n_out) {
+    __shared__ bf16 tile[32][kInPad + 2];
+    const int r0 = blockIdx.x * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = *step + 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) loss[t] = 0.0f;
+    const uint4 u = philox4x32_10(make_uint4((uint32_t)(r0 + lane), (uint32_t)t, 0x6d6c70u, 0u), k0, k1);
+    const int own = (int)(((unsigned long long)u.x * (unsigned long long)ds_rows) >> 32);
+    if (warp == 0) src[r0 + lane] = own;
+    // the targets come into L2 while the hidden layers run; the output layer's epilogue, which would wait for
+    // DRAM at every line, then finds them there (42 -> 20 us of that layer at 4,096 rows)
+    for (int k = warp; k < 32; k += 8) {
+        const float* tp = ds_t + (size_t)__shfl_sync(0xffffffffu, own, k) * n_out;
+        for (int c = 32 * lane; c < n_out; c += 32 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(tp + c));
+        if (lane == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(tp + n_out - 1));
+    }
+    for (int k = warp; k < 32; k += 8) {
+        const int s = __shfl_sync(0xffffffffu, own, k);
+        const uint32_t v = reinterpret_cast<const uint32_t*>(ds_x + (size_t)s * kInPad)[lane];
+        reinterpret_cast<uint32_t*>(xb + (size_t)(r0 + k) * kInPad)[lane] = v;
+        *reinterpret_cast<uint32_t*>(&tile[k][2 * lane]) = v;
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < kInPad; c += blockDim.x) {
-        const bf16 v = ds_x[(size_t)src * kInPad + c];
-        xb[(size_t)r * kInPad + c] = v;
-        xt[(size_t)c * rows + r] = v;
+    for (int c = warp; c < kInPad; c += 8) xt[(size_t)c * rows + r0 + lane] = tile[lane][c];
+}
+
+// db of one unit: the sum over the rows of dZ^T, by a warp. 256 running sums (eight per lane, row r in sum
+// r % 256), then their pairwise tree: a fixed order, whatever the launch.
+__device__ __forceinline__ float bias_grad(const bf16* __restrict__ dzt_row, int rows, int lane) {
+    float s[8] = {};
+#pragma unroll 4
+    for (int i = 0; i < rows; i += 256) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (i + 32 * k < rows) s[k] += __bfloat162float(dzt_row[i + 32 * k + lane]);
     }
-    for (int c = threadIdx.x; c < n_out; c += blockDim.x) tb[(size_t)r * n_out + c] = ds_t[(size_t)src * n_out + c];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < o; ++k) s[k] += s[k + o];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[0] += __shfl_down_sync(0xffffffffu, s[0], o);
+    return s[0];  // lane 0's
 }
-
-__global__ void step_kernel(int* step, float* loss) {
-    *step += 1;
-    loss[*step] = 0.0f;
-}
-
-// db[n] = sum over rows of dZ^T[n][row] (fixed order: deterministic)
 __global__ void bias_grad_kernel(const bf16* __restrict__ dzt, int rows, float* __restrict__ db) {
-    const int n = blockIdx.x;
-    float s = 0.0f;
-    for (int i = threadIdx.x; i < rows; i += blockDim.x) s += __bfloat162float(dzt[(size_t)n * rows + i]);
-    __shared__ float red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) db[n] = red[0];
+    const int n = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const float s = bias_grad(dzt + (size_t)n * rows, rows, lane);
+    if (lane == 0) db[n] = s;
 }
 
 // g[i] = sum over splits of part[s][i] (fixed order)
@@ -247,32 +304,89 @@ __global__ void split_sum_kernel(const float* __restrict__ part, int splits, siz
     }
 }
 
-// Adam (Kingma & Ba, 2015) on FP32 master parameters p[rows x cols] with bias correction from the
-// step counter; refreshes the bf16 copy (row-major) and its transpose when given.
-__global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                            int rows, int cols, int valid_rows, float lr, float b1, float b2, float eps,
-                            const int* __restrict__ step, bf16* __restrict__ w16, bf16* __restrict__ w16t) {
-    const size_t n = (size_t)rows * cols;
-    const int t = *step;
-    const float c1 = 1.0f - __powf(b1, (float)t), c2 = 1.0f - __powf(b2, (float)t);
-    const float alpha = lr * sqrtf(c2) / c1;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / cols), c = (int)(i % cols);
-        float w = p[i];
-        if (r < valid_rows) {
-            const float gi = g[i];
-            const float mi = b1 * m[i] + (1.0f - b1) * gi;
-            const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-            m[i] = mi;
-            v[i] = vi;
-            w -= alpha * mi / (sqrtf(vi) + eps);
-            p[i] = w;
+// One Adam step (Kingma & Ba, 2015) on one FP32 master parameter and its moments, bias correction in alpha.
+__device__ __forceinline__ float adam(float w, float g, float& m, float& v, float alpha, float b1, float b2, float eps) {
+    m = b1 * m + (1.0f - b1) * g;
+    v = b2 * v + (1.0f - b2) * g * g;
+    return w - alpha * m / (sqrtf(v) + eps);
+}
+
+struct UpdateLayer {
+    float *w, *m, *v, *b, *mb, *vb;  // masters and moments of the weights [rows x cols] and biases [rows]
+    const float* part;               // [splits][rows x cols] partial weight gradients
+    const float* gb;                 // [rows] bias gradients
+    bf16 *w16, *w16t;
+    int rows, cols, valid_rows, splits;
+    int first_tile, first_bias;      // its first block of weights and of biases in the launch
+};  // (blocks of 256 biases)
+struct UpdateParams {
+    UpdateLayer layer[kMaxLayers];
+    int layers, biases;              // the first `biases` blocks take biases, the others weights
+    float lr, b1, b2, eps;
+    int *step, *ticket;
+};
+
+// Gradient sums and Adam of every parameter of the network in one launch: blocks of 32 x 32 weights sum their
+// split-K partials in split order, step, and write the bf16 copies both ways through a shared tile; the
+// last block to finish counts the step. As four launches per layer (split sums, bias sums, two Adam launches
+// with strided transposed stores) this took 130 us of a 296 us step on a 15-256x4-1000 network at 4,096 rows;
+// now 44 us, bound by the partials (71 MB, written and read back), with the bias sums beside the backward
+// chain. Folding the splits in one CTA per tile instead, in the same order, moved no time: 64 dependent
+// k-blocks took 36 us per layer and what they saved here (144 us per step against 150, slower at 8,192 rows).
+__global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ UpdateParams P) {
+    const int t = *P.step + 1;
+    const float c1 = 1.0f - __powf(P.b1, (float)t), c2 = 1.0f - __powf(P.b2, (float)t);
+    const float alpha = P.lr * sqrtf(c2) / c1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int l = P.layers - 1;
+    if ((int)blockIdx.x >= P.biases) {
+        const int blk = (int)blockIdx.x - P.biases;
+        while (blk < P.layer[l].first_tile) --l;
+        const UpdateLayer& L = P.layer[l];
+        const int tile = blk - L.first_tile, tc = L.cols / 32;
+        const int r0 = tile / tc * 32, c0 = tile % tc * 32;
+        const size_t n = (size_t)L.rows * L.cols;
+        __shared__ bf16 s[32][33];
+        // every load of the thread's four weights before the first store
+        const size_t i0 = (size_t)(r0 + warp) * L.cols + c0 + lane, di = 8 * (size_t)L.cols;
+        float w[4], m[4], v[4], g[4] = {};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            w[k] = L.w[i0 + k * di];
+            m[k] = L.m[i0 + k * di];
+            v[k] = L.v[i0 + k * di];
         }
-        if (w16) {
-            const bf16 h = __float2bfloat16_rn(w);
-            w16[i] = h;
-            w16t[(size_t)c * rows + r] = h;
+#pragma unroll 8
+        for (int q = 0; q < L.splits; ++q)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) g[k] += __ldg(&L.part[(size_t)q * n + i0 + k * di]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (r0 + warp + 8 * k < L.valid_rows) {
+                w[k] = adam(w[k], g[k], m[k], v[k], alpha, P.b1, P.b2, P.eps);
+                L.m[i0 + k * di] = m[k];
+                L.v[i0 + k * di] = v[k];
+                L.w[i0 + k * di] = w[k];
+            }
+            const bf16 h = __float2bfloat16_rn(w[k]);
+            L.w16[i0 + k * di] = h;
+            s[warp + 8 * k][lane] = h;
         }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) L.w16t[(size_t)(c0 + warp + 8 * k) * L.rows + r0 + lane] = s[lane][warp + 8 * k];
+    } else {
+        const int blk = (int)blockIdx.x;
+        while (blk < P.layer[l].first_bias) --l;
+        const UpdateLayer& L = P.layer[l];
+        const int r = (blk - L.first_bias) * 256 + threadIdx.x;
+        if (r < L.valid_rows) L.b[r] = adam(L.b[r], L.gb[r], L.mb[r], L.vb[r], alpha, P.b1, P.b2, P.eps);
+    }
+    // every block has read *step before it takes its ticket
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(P.ticket, 1) == (int)gridDim.x - 1) {
+        *P.ticket = 0;
+        *P.step = t;
     }
 }
 
@@ -410,8 +524,10 @@ struct xmc_mlp {
     bf16 *dz[kMaxLayers] = {}, *dzt[kMaxLayers] = {};
     float *y = nullptr, *t = nullptr, *xin = nullptr;
     float* colw = nullptr;          // per-output loss weights, or null
-    float* part = nullptr;
-    size_t part_floats = 0;
+    float* part[kMaxLayers] = {};   // split-K partials of each layer's weight gradient (one allocation, part[0])
+    int* src = nullptr;             // minibatch rows' places in the data set
+    cudaStream_t side[2] = {};      // weight gradients beside the data gradients, layers in turn
+    cudaEvent_t ev_dz[kMaxLayers] = {}, ev_side[2] = {};
     // data set
     bf16* ds_x = nullptr;
     float* ds_t = nullptr;
@@ -434,7 +550,7 @@ void free_mlp(xmc_mlp* m) {
     cudaSetDevice(m->spec.device);
     for (auto& kv : m->train_graphs) cudaGraphExecDestroy(kv.second);
     for (auto& kv : m->fwd_graphs) cudaGraphExecDestroy(kv.second);
-    std::vector<void*> d = {m->d_err, m->d_step, m->d_loss, m->x, m->xt, m->y, m->t, m->xin, m->part, m->ds_x, m->ds_t,
+    std::vector<void*> d = {m->d_err, m->d_step, m->d_loss, m->x, m->xt, m->y, m->t, m->xin, m->src, m->part[0], m->ds_x, m->ds_t,
                             m->colw};
     for (int l = 0; l < kMaxLayers; ++l)
         for (void* p : {(void*)m->w32[l], (void*)m->b32[l], (void*)m->mw[l], (void*)m->vw[l], (void*)m->mb[l],
@@ -448,11 +564,24 @@ void free_mlp(xmc_mlp* m) {
     if (m->h_y) cudaFreeHost(m->h_y);
     for (cudaEvent_t e : m->ev_chunk)
         if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : m->ev_dz)
+        if (e) cudaEventDestroy(e);
+    for (int k = 0; k < 2; ++k) {
+        if (m->ev_side[k]) cudaEventDestroy(m->ev_side[k]);
+        if (m->side[k]) cudaStreamDestroy(m->side[k]);
+    }
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
 }
 
-// split-K factor of the weight-gradient GEMM of layer l for `rows` rows: about 128 CTAs
+// Widest tile that still gives the chip's SMs a CTA each, else the narrowest: the tile width changes no sum.
+int tile_width(int rows_a, int n, int splits) {
+    for (int bn = 256; bn > 64; bn /= 2)
+        if (n % bn == 0 && (rows_a / tc::kBM) * (n / bn) * splits >= 148) return bn;
+    return 64;
+}
+
+// split-K factor of the weight-gradient GEMM of layer l for `rows` rows: about 128 CTAs of full width
 int wgrad_splits(const xmc_mlp* m, int l, int rows) {
     const int tiles = m->out[l] / tc::kBM;
     const int kblocks = rows / tc::kBK;
@@ -496,8 +625,20 @@ int enqueue_fused_forward(xmc_mlp* m, int rows) {
     return XMC_OK;
 }
 
-// Forward pass over `rows` rows of m->x (bf16, padded). Training: also Z, A^T, dY, loss.
-int enqueue_forward(xmc_mlp* m, int rows, bool train) {
+// D = A . B^T with the widest tile that fills the chip.
+template <class Epi>
+int launch_gemm_wide(const void* a, int rows_a, const void* b, int n, int k, int splits, const Epi& epi, int* err,
+                     cudaStream_t stream) {
+    switch (tile_width(rows_a, n, splits)) {
+        case 256: return launch_gemm<256>(a, rows_a, b, n, k, splits, epi, err, stream);
+        case 128: return launch_gemm<128>(a, rows_a, b, n, k, splits, epi, err, stream);
+        default: return launch_gemm<64>(a, rows_a, b, n, k, splits, epi, err, stream);
+    }
+}
+
+// Forward pass over `rows` rows of m->x (bf16, padded). Training: also Z, A^T, dY, loss, with the targets from
+// m->t or, for a minibatch, from the data set.
+int enqueue_forward(xmc_mlp* m, int rows, bool train, bool from_data_set = false) {
     if (!train && fused_forward_ok(m)) return enqueue_fused_forward(m, rows);
     const cudaStream_t st = m->stream;
     for (int l = 0; l < m->L; ++l) {
@@ -506,15 +647,16 @@ int enqueue_forward(xmc_mlp* m, int rows, bool train) {
         int s;
         if (l < m->L - 1) {
             EpiHidden e{m->b32[l], m->a[l], m->out[l], train ? m->z[l] : nullptr, train ? m->at[l] : nullptr, rows};
-            s = m->out[l] == 256 ? launch_gemm<256>(a_in, rows, m->w16[l], m->out[l], k, 1, e, m->d_err, st)
-                                 : launch_gemm<128>(a_in, rows, m->w16[l], m->out[l], k, 1, e, m->d_err, st);
+            s = launch_gemm_wide(a_in, rows, m->w16[l], m->out[l], k, 1, e, m->d_err, st);
         } else {
             EpiOut e{};
             e.bias = m->b32[l];
             e.n_out = m->spec.n_out;
             if (train) {
                 e.y = nullptr;
-                e.t = m->t;
+                e.t = from_data_set ? m->ds_t : m->t;
+                e.src = from_data_set ? m->src : nullptr;
+                e.step_add = from_data_set ? 1 : 0;  // the step under way is counted when it is done
                 e.ldtg = m->spec.n_out;
                 e.dy = m->dz[l];
                 e.lddy = m->out[l];
@@ -528,49 +670,87 @@ int enqueue_forward(xmc_mlp* m, int rows, bool train) {
                 e.y = m->y;
                 e.ldy = m->spec.n_out;
             }
-            s = launch_gemm<256>(a_in, rows, m->w16[l], m->out[l], k, 1, e, m->d_err, st);
+            s = launch_gemm_wide(a_in, rows, m->w16[l], m->out[l], k, 1, e, m->d_err, st);
         }
         if (s) return s;
     }
     return XMC_OK;
 }
 
-// Backward pass after enqueue_forward(train): gradients into gw / gb.
+// What training alone needs, on the first call that trains: streams and events of the backward pass, the
+// minibatch's row numbers, and the split-K partials of every layer at the largest split any batch takes.
+int ensure_training(xmc_mlp* m) {
+    if (m->part[0]) return XMC_OK;
+    for (int k = 0; k < 2; ++k) {
+        if (!m->side[k]) XM_CUDA(cudaStreamCreateWithFlags(&m->side[k], cudaStreamNonBlocking));
+        if (!m->ev_side[k]) XM_CUDA(cudaEventCreateWithFlags(&m->ev_side[k], cudaEventDisableTiming));
+    }
+    size_t floats[kMaxLayers + 1] = {};
+    for (int l = 0; l < m->L; ++l) {
+        if (!m->ev_dz[l]) XM_CUDA(cudaEventCreateWithFlags(&m->ev_dz[l], cudaEventDisableTiming));
+        floats[l + 1] = floats[l] + (size_t)m->out[l] * m->in[l] * std::max(1, 128 / (m->out[l] / tc::kBM));
+    }
+    if (!m->src) XM_CUDA(cudaMalloc(&m->src, sizeof(int) * (size_t)m->cap));
+    XM_CUDA(cudaMalloc(&m->part[0], sizeof(float) * floats[m->L]));
+    for (int l = 1; l < m->L; ++l) m->part[l] = m->part[0] + floats[l];
+    return XMC_OK;
+}
+
+// Backward pass after enqueue_forward(train): per-layer partial weight gradients into m->part, bias gradients
+// into m->gb. The data gradients are one chain; each layer's weight and bias gradients hang off it and run on
+// a stream of their own.
 int enqueue_backward(xmc_mlp* m, int rows) {
     const cudaStream_t st = m->stream;
     for (int l = m->L - 1; l >= 0; --l) {
-        // data gradient to the previous layer
+        XM_CUDA(cudaEventRecord(m->ev_dz[l], st));  // dZ_l is ready
         if (l > 0) {
             EpiBwd e{m->z[l - 1], m->out[l - 1], m->dz[l - 1], m->dzt[l - 1], rows};
-            int s = m->in[l] == 256 ? launch_gemm<256>(m->dz[l], rows, m->w16t[l], m->in[l], m->out[l], 1, e, m->d_err, st)
-                                    : launch_gemm<128>(m->dz[l], rows, m->w16t[l], m->in[l], m->out[l], 1, e, m->d_err, st);
+            const int s = launch_gemm_wide(m->dz[l], rows, m->w16t[l], m->in[l], m->out[l], 1, e, m->d_err, st);
             if (s) return s;
         }
-        // weight gradient: dW = dZ^T . A_{l-1}, split over rows
-        const int splits = wgrad_splits(m, l, rows);
-        const bf16* bt = l == 0 ? m->xt : m->at[l - 1];
-        const size_t n = (size_t)m->out[l] * m->in[l];
-        EpiF32 e{m->part, m->in[l], n};
-        int s;
-        if (m->in[l] == 256) s = launch_gemm<256>(m->dzt[l], m->out[l], bt, m->in[l], rows, splits, e, m->d_err, st);
-        else if (m->in[l] == 128) s = launch_gemm<128>(m->dzt[l], m->out[l], bt, m->in[l], rows, splits, e, m->d_err, st);
-        else s = launch_gemm<64>(m->dzt[l], m->out[l], bt, m->in[l], rows, splits, e, m->d_err, st);
-        if (s) return s;
-        split_sum_kernel<<<296, 256, 0, st>>>(m->part, splits, n, m->gw[l]);
-        bias_grad_kernel<<<m->out[l], 256, 0, st>>>(m->dzt[l], rows, m->gb[l]);
+        // bias gradient, then the weight gradient dW = dZ^T . A_{l-1}, split over rows. The first layer's, the last
+        // to start, run side by side.
+        XM_CUDA(cudaStreamWaitEvent(m->side[l & 1], m->ev_dz[l], 0));
+        bias_grad_kernel<<<m->out[l] / 8, 256, 0, l > 0 ? m->side[l & 1] : st>>>(m->dzt[l], rows, m->gb[l]);
         XM_CUDA(cudaGetLastError());
+        const bf16* bt = l == 0 ? m->xt : m->at[l - 1];
+        EpiF32 e{m->part[l], m->in[l], (size_t)m->out[l] * m->in[l]};
+        const int s = launch_gemm_wide(m->dzt[l], m->out[l], bt, m->in[l], rows, wgrad_splits(m, l, rows), e, m->d_err, m->side[l & 1]);
+        if (s) return s;
+    }
+    for (int k = 0; k < std::min(2, m->L); ++k) {
+        XM_CUDA(cudaEventRecord(m->ev_side[k], m->side[k]));
+        XM_CUDA(cudaStreamWaitEvent(st, m->ev_side[k], 0));
     }
     return XMC_OK;
 }
 
-int enqueue_adam(xmc_mlp* m, float lr, float b1, float b2, float eps) {
-    const cudaStream_t st = m->stream;
+// Sums of the weight gradients after enqueue_backward, into gw.
+int enqueue_gradient_sums(xmc_mlp* m, int rows) {
     for (int l = 0; l < m->L; ++l) {
-        adam_kernel<<<296, 256, 0, st>>>(m->w32[l], m->gw[l], m->mw[l], m->vw[l], m->out[l], m->in[l], m->valid_out[l], lr, b1,
-                                         b2, eps, m->d_step, m->w16[l], m->w16t[l]);
-        adam_kernel<<<8, 256, 0, st>>>(m->b32[l], m->gb[l], m->mb[l], m->vb[l], m->out[l], 1, m->valid_out[l], lr, b1, b2,
-                                       eps, m->d_step, nullptr, nullptr);
+        split_sum_kernel<<<296, 256, 0, m->stream>>>(m->part[l], wgrad_splits(m, l, rows), (size_t)m->out[l] * m->in[l], m->gw[l]);
     }
+    XM_CUDA(cudaGetLastError());
+    return XMC_OK;
+}
+
+// Gradient sums and Adam after enqueue_backward.
+int enqueue_update(xmc_mlp* m, int rows, float lr, float b1, float b2, float eps) {
+    UpdateParams p;
+    std::memset(&p, 0, sizeof(p));
+    int tiles = 0;
+    for (int l = 0; l < m->L; ++l) {
+        UpdateLayer& U = p.layer[l];
+        U = {m->w32[l], m->mw[l], m->vw[l], m->b32[l], m->mb[l], m->vb[l], m->part[l], m->gb[l], m->w16[l], m->w16t[l],
+             m->out[l], m->in[l], m->valid_out[l], wgrad_splits(m, l, rows), tiles, p.biases};
+        tiles += m->out[l] / 32 * (m->in[l] / 32);
+        p.biases += (m->out[l] + 255) / 256;
+    }
+    p.layers = m->L;
+    p.lr = lr; p.b1 = b1; p.b2 = b2; p.eps = eps;
+    p.step = m->d_step;
+    p.ticket = m->d_step + 1;
+    update_kernel<<<tiles + p.biases, 256, 0, m->stream>>>(p);
     XM_CUDA(cudaGetLastError());
     return XMC_OK;
 }
@@ -639,13 +819,12 @@ extern "C" int xmc_mlp_create(const xmc_mlp_spec* spec, xmc_mlp** out) {
     XM_TRY(cudaEventCreate(&m->ev[0]));
     XM_TRY(cudaEventCreate(&m->ev[1]));
     XM_TRY(cudaMalloc(&m->d_err, sizeof(int)));
-    XM_TRY(cudaMalloc(&m->d_step, sizeof(int)));
+    XM_TRY(cudaMalloc(&m->d_step, 2 * sizeof(int)));  // steps taken, tickets of the step under way
     m->loss_cap = 1 << 20;
     XM_TRY(cudaMalloc(&m->d_loss, sizeof(float) * (m->loss_cap + 1)));
     XM_TRY(cudaMemset(m->d_err, 0, sizeof(int)));
-    XM_TRY(cudaMemset(m->d_step, 0, sizeof(int)));
+    XM_TRY(cudaMemset(m->d_step, 0, 2 * sizeof(int)));
     const size_t R = (size_t)m->cap;
-    size_t part = 0;
     for (int l = 0; l < m->L; ++l) {
         const size_t n = (size_t)m->out[l] * m->in[l];
         XM_TRY(cudaMalloc(&m->w32[l], sizeof(float) * n));
@@ -667,12 +846,7 @@ extern "C" int xmc_mlp_create(const xmc_mlp_spec* spec, xmc_mlp** out) {
         XM_TRY(cudaMalloc(&m->z[l], sizeof(bf16) * R * m->out[l]));
         XM_TRY(cudaMalloc(&m->dz[l], sizeof(bf16) * R * m->out[l]));
         XM_TRY(cudaMalloc(&m->dzt[l], sizeof(bf16) * R * m->out[l]));
-        // largest split-K partial buffer over the batch sizes this model can take
-        const int tiles = m->out[l] / tc::kBM;
-        part = std::max(part, (size_t)std::max(1, 128 / tiles) * n);
     }
-    m->part_floats = part;
-    XM_TRY(cudaMalloc(&m->part, sizeof(float) * part));
     XM_TRY(cudaMalloc(&m->x, sizeof(bf16) * R * kInPad));
     XM_TRY(cudaMalloc(&m->xt, sizeof(bf16) * R * kInPad));
     XM_TRY(cudaMalloc(&m->xin, sizeof(float) * R * s.n_in));
@@ -864,7 +1038,8 @@ extern "C" int xmc_mlp_gradients(xmc_mlp* m, const float* x, const float* t, int
     int st = check_rows(m, rows);
     if (st) return st;
     XM_CUDA(cudaSetDevice(m->spec.device));
-    st = upload_inputs(m, x, rows, true);
+    st = ensure_training(m);
+    if (!st) st = upload_inputs(m, x, rows, true);
     if (st) return st;
     XM_CUDA(cudaMemcpyAsync(m->t, t, sizeof(float) * (size_t)rows * m->spec.n_out, cudaMemcpyHostToDevice, m->stream));
     // loss slot: loss[step + ... ] uses *d_step; use slot (current step) after zeroing it
@@ -875,6 +1050,7 @@ extern "C" int xmc_mlp_gradients(xmc_mlp* m, const float* x, const float* t, int
     st = enqueue_forward(m, rows, true);
     if (st) return st;
     st = enqueue_backward(m, rows);
+    if (!st) st = enqueue_gradient_sums(m, rows);
     if (st) return st;
     float l = 0.0f;
     XM_CUDA(cudaMemcpyAsync(&l, m->d_loss + step, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
@@ -889,6 +1065,9 @@ extern "C" int xmc_mlp_set_dataset(xmc_mlp* m, const float* x, const float* t, i
     xmc::DeviceGuard device_guard;  // the caller's current device is restored on return
     if (!m || !x || !t || rows < 1) return mfail(XMC_ERR_INVALID_INPUT, "NULL argument or empty data set");
     XM_CUDA(cudaSetDevice(m->spec.device));
+    XM_CUDA(cudaStreamSynchronize(m->stream));
+    for (auto& kv : m->train_graphs) cudaGraphExecDestroy(kv.second);  // they hold the old data set's addresses
+    m->train_graphs.clear();
     if (m->ds_x) cudaFree(m->ds_x);
     if (m->ds_t) cudaFree(m->ds_t);
     m->ds_x = nullptr;
@@ -921,6 +1100,8 @@ extern "C" int xmc_mlp_train(xmc_mlp* m, int steps, int batch, float lr, float b
     int st = check_rows(m, batch);
     if (st) return st;
     XM_CUDA(cudaSetDevice(m->spec.device));
+    st = ensure_training(m);
+    if (st) return st;
     int step0 = 0;
     XM_CUDA(cudaMemcpy(&step0, m->d_step, sizeof(int), cudaMemcpyDeviceToHost));
     if (step0 + steps >= m->loss_cap) return mfail(XMC_ERR_RANGE, "too many training steps for the loss log");
@@ -935,12 +1116,12 @@ extern "C" int xmc_mlp_train(xmc_mlp* m, int steps, int batch, float lr, float b
         ex = it->second;
     } else {
         XM_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
-        step_kernel<<<1, 1, 0, m->stream>>>(m->d_step, m->d_loss);
-        gather_kernel<<<batch, 128, 0, m->stream>>>(m->ds_x, m->ds_t, m->ds_rows, m->spec.n_out, batch, (uint32_t)seed,
-                                                    (uint32_t)(seed >> 32), m->d_step, m->x, m->xt, m->t);
-        st = enqueue_forward(m, batch, true);
+        gather_kernel<<<batch / 32, 256, 0, m->stream>>>(m->ds_x, m->ds_rows, batch, (uint32_t)seed, (uint32_t)(seed >> 32),
+                                                         m->d_step, m->d_loss, m->x, m->xt, m->src, m->ds_t,
+                                                         m->spec.n_out);
+        st = enqueue_forward(m, batch, true, true);
         if (!st) st = enqueue_backward(m, batch);
-        if (!st) st = enqueue_adam(m, lr, beta1, beta2, eps);
+        if (!st) st = enqueue_update(m, batch, lr, beta1, beta2, eps);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(m->stream, &g);
         if (st) {

@@ -4,7 +4,7 @@
 //
 // One CTA of 256 threads computes a 128 x BN tile of D over a range of K (split-K when the grid's
 // z extent is > 1). Operand tiles of 128 (A) and BN (B) rows x 64 bf16 (128 B) are brought into
-// shared memory by TMA (cp.async.bulk.tensor.2d, 128-byte swizzle) through a 2-stage ring of
+// shared memory by TMA (cp.async.bulk.tensor.2d, 128-byte swizzle) through a 2- to 4-stage ring of
 // mbarrier-tracked buffers; one thread issues the tcgen05.mma instructions (M = 128, N = BN,
 // K = 16 each, both operands K-major, read from shared memory through matrix descriptors) into a
 // TMEM accumulator of BN columns, and tcgen05.commit signals the ring's "empty" barriers and the
@@ -26,12 +26,13 @@ namespace tc {
 constexpr int kBM = 128;          // tile rows (MMA M)
 constexpr int kThreads = 256;     // 8 warps: warp w reads TMEM lanes 32 (w % 4).., column half w / 4
 constexpr int kBK = 64;           // K per stage: 64 bf16 = one 128-byte swizzle row
-constexpr int kStages = 2;  // small enough that two CTAs (BN = 256) share an SM: one's epilogue
-                              // overlaps the other's loads and MMAs
+// Ring stages: 96 KB for every tile width, so that two CTAs share an SM (one's epilogue overlaps the other's
+// loads and MMAs); a narrow tile's k-blocks take less time than a TMA round trip and need more in flight.
+__host__ __device__ constexpr int stages(int bn) { return bn == 64 ? 4 : bn == 128 ? 3 : 2; }
 constexpr unsigned long long kWaitNs = 2000000000ull;  // bound of any single pipeline wait: 2 s
 
 __host__ __device__ constexpr int stage_bytes(int bn) { return (kBM + bn) * kBK * 2; }
-__host__ __device__ constexpr int smem_bytes(int bn) { return kStages * stage_bytes(bn) + 1024 + 256; }
+__host__ __device__ constexpr int smem_bytes(int bn) { return stages(bn) * stage_bytes(bn) + 1024 + 256; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -136,6 +137,7 @@ template <int BN, class Epi>
 __global__ void __launch_bounds__(kThreads, 2)
     gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int k_blocks_per_split,
                 int* err, const Epi epi) {
+    constexpr int kStages = stages(BN);
     static_assert(BN == 64 || BN == 128 || BN == 256, "BN");
     static_assert(kStages * stage_bytes(BN) >= (kThreads / 32) * 32 * 33 * 4, "epilogue staging tiles fit the ring");
     extern __shared__ unsigned char smem_raw[];
