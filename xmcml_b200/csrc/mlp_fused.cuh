@@ -1,6 +1,7 @@
 // Fused forward pass (inference) of the surrogate MLP on the sm_100a tensor cores.
 //
-// One persistent CTA per SM walks its 128-row tiles of the input two at a time, in two slots. For each
+// One persistent CTA per SM walks its 128-row tiles of the input two at a time, in two slots (one slot when
+// there are no more tiles than SMs). For each
 // tile every layer runs in turn with the tile's activations kept in the slot's shared-memory buffer H,
 // so nothing but the inputs, the weights (L2-resident, streamed by TMA) and the FP32 outputs touches
 // global memory:
@@ -35,11 +36,13 @@ namespace xmc {
 namespace fused {
 
 constexpr int kMaxL = 9;
-constexpr int kSlots = 2;     // tiles in flight per CTA
+constexpr int kMaxSlots = 2;  // tiles in flight per CTA
 constexpr int kEpiWarps = 16;  // warp w reads TMEM lanes 32 (w % 4).. and column quarter w / 4
 constexpr int kColGroups = kEpiWarps / 4;
 constexpr int kThreads = 32 * (kEpiWarps + 2);
-constexpr int kWStages = 2;                // weight ring depth (stages of 64 K-columns)
+constexpr int kMaxWStages = 4;
+// weight ring depth (stages of 64 K-columns): the second slot's activations make room for two more stages
+__host__ __device__ constexpr int w_stages(int slots) { return slots == 1 ? 4 : 2; }
 constexpr int kXBytes = 128 * 64 * 2;      // input tile, one 64-column k-block
 constexpr int kKBlockBytes = 128 * 128;    // one 64-column k-block of a 128-row operand
 constexpr int kHBytes = 4 * kKBlockBytes;  // activations of one slot, hidden <= 256
@@ -48,8 +51,8 @@ constexpr int kOutCols = 16;               // columns of one output box (64 byte
 constexpr int kOutBox = 32 * kOutCols * 4; // one warp's 32 x 16 FP32 output box
 constexpr int kOutBufs = 1;                // output staging boxes per epilogue warp
 constexpr int kOffH = 0;
-constexpr int kOffW = kOffH + kSlots * kHBytes;
-constexpr int kOffO = kOffW + kWStages * kWBytes;
+constexpr int kOffO = kOffH + kMaxSlots * kHBytes + 2 * kWBytes;
+static_assert(kHBytes + 4 * kWBytes <= kOffO, "one slot and four weight stages take what two and two take");
 constexpr int kOffBar = kOffO + kEpiWarps * kOutBufs * kOutBox;
 constexpr int kSmemBytes = kOffBar + 256 + 1024;  // barriers, TMEM slot, abort flag; alignment slack
 static_assert(kSmemBytes <= 232448, "fused forward exceeds the shared memory of one CTA");
@@ -65,6 +68,7 @@ struct Params {
     int out_chunks;            // padded output columns / 256
     int n_tiles;               // rows / 128
     int n_out;                 // output columns (boxes past them are not stored)
+    int split;                 // 1: a CTA computes one output chunk of one tile (CTA = tile x chunk)
     int* err;
 };
 
@@ -101,7 +105,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 
 // layer geometry: MMA N of one chunk, chunks, 64-column k-blocks
 __device__ __forceinline__ int layer_n(const Params& p, int l) { return l < p.L - 1 ? p.hidden : 256; }
-__device__ __forceinline__ int layer_chunks(const Params& p, int l) { return l < p.L - 1 ? 1 : p.out_chunks; }
+__device__ __forceinline__ int layer_chunks(const Params& p, int l) { return l < p.L - 1 || p.split ? 1 : p.out_chunks; }
 __device__ __forceinline__ int layer_kblocks(const Params& p, int l) { return l == 0 ? 1 : p.hidden / 64; }
 
 // Epilogue of 32 accumulator columns of a hidden layer: bias + SiLU, written as BF16 (4 chunks of 16 B)
@@ -189,9 +193,9 @@ struct JobOrder {
         s = a0 && a1 ? turn : (a0 ? 0 : 1);
         turn = s ^ 1;
         int i = s ? i1 : i0, l = s ? l1 : l0, c = s ? c1 : c0;
-        tile = (int)blockIdx.x + i * (int)gridDim.x;
+        tile = p.split ? (int)blockIdx.x / p.out_chunks : (int)blockIdx.x + i * (int)gridDim.x;
         layer = l;
-        chunk = c;
+        chunk = p.split && l == p.L - 1 ? (int)blockIdx.x % p.out_chunks : c;
         if (++c == layer_chunks(p, l)) {
             c = 0;
             if (++l == p.L) l = 0, i += 2;
@@ -202,7 +206,13 @@ struct JobOrder {
     }
 };
 
+// kSlots == 1: at most one tile per CTA (few rows). Such a launch is bound by the latency of a tile's chain of
+// layers, and that by the weight stream: with two stages a CTA has 64 KB on their way per L2 round trip. One
+// slot leaves room for four; with `split` a CTA also takes only one of the output chunks (hidden layers are
+// computed by each of them). 15-256x4-1000, 128 rows: 36 -> 22.6 us (8,192 rows, no split: 36.9 -> 35.1).
+template <int kSlots>
 __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_constant__ Params p) {
+    constexpr int kWStages = w_stages(kSlots), kOffW = kOffH + kSlots * kHBytes;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = tc::smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -210,8 +220,9 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
     const uint32_t sH = base + kOffH, sW = base + kOffW, sO = base + kOffO;
     const uint32_t bar = base + kOffBar;
     // two of each per slot (or per ring stage), 8 bytes apart
-    const uint32_t w_full = bar, w_empty = bar + 16, x_full = bar + 32, x_empty = bar + 48;
+    const uint32_t x_full = bar + 32, x_empty = bar + 48;
     const uint32_t acc_full = bar + 64, acc_empty = bar + 80, h_full = bar + 96, drain = bar + 112;
+    const uint32_t w_full = bar + 120, w_empty = w_full + 8 * kMaxWStages;  // up to bar + 184
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(gbase + kOffBar + 192);
     volatile int* s_abort = reinterpret_cast<volatile int*>(gbase + kOffBar + 196);
 
@@ -221,9 +232,11 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
         tc::tmem_relinquish();
     }
     if (threadIdx.x == 32 * kEpiWarps) {
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < kWStages; ++s) {
             tc::mbar_init(w_full + 8 * s, 1);
             tc::mbar_init(w_empty + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; ++s) {
             tc::mbar_init(x_full + 8 * s, 1);
             tc::mbar_init(x_empty + 8 * s, 1);
             tc::mbar_init(acc_full + 8 * s, 1);
@@ -239,7 +252,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
     tc::tc_fence_after();
     const uint32_t taddr = *s_tmem;
     // this CTA's tiles are blockIdx.x + i gridDim.x, i < my_tiles (JobOrder deals them to the slots)
-    const int my_tiles = (p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int my_tiles = p.split ? 1 : (p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
     if (warp == kEpiWarps && lane == 0) {
         // ---------------- TMA producer ----------------
@@ -284,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
             const uint32_t idesc = l < p.L - 1 ? idesc_h : idesc_o;
             if (!(ok = tc::mbar_wait(acc_empty + 8 * s, (ja.get(s) & 1) ^ 1, p.err))) break;
             if (l == 0) ok = tc::mbar_wait(x_full + 8 * s, xm.take(s) & 1, p.err);
-            else if (c == 0) ok = tc::mbar_wait(h_full + 8 * s, hw.take(s) & 1, p.err);
+            else if (p.split || c == 0) ok = tc::mbar_wait(h_full + 8 * s, hw.take(s) & 1, p.err);
             if (!ok || *s_abort) { ok = false; break; }
             tc::tc_fence_after();
             const uint32_t d = taddr + 256u * s, a0 = sH + s * kHBytes;
@@ -300,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
             }
             if (!ok) break;
             // the slot's last MMAs of this tile: its activations may take the next X tile
-            if (l == p.L - 1 && c == nc - 1) tc::umma_commit(x_empty + 8 * s);
+            if (l == p.L - 1 && (p.split || c == nc - 1)) tc::umma_commit(x_empty + 8 * s);
             tc::umma_commit(acc_full + 8 * s);
             ja.take(s);
         }

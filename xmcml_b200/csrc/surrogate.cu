@@ -598,7 +598,9 @@ bool fused_forward_ok(const xmc_mlp* m) {
 int enqueue_fused_forward(xmc_mlp* m, int rows) {
     static bool attr = false;
     if (!attr) {
-        XM_CUDA(cudaFuncSetAttribute(fused::mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        XM_CUDA(cudaFuncSetAttribute(fused::mlp_forward_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     fused::kSmemBytes));
+        XM_CUDA(cudaFuncSetAttribute(fused::mlp_forward_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      fused::kSmemBytes));
         attr = true;
     }
@@ -619,8 +621,13 @@ int enqueue_fused_forward(xmc_mlp* m, int rows) {
     p.err = m->d_err;
     int sms = 0;
     XM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->spec.device));
-    const int grid = std::min(p.n_tiles, sms);
-    fused::mlp_forward_kernel<<<grid, fused::kThreads, fused::kSmemBytes, m->stream>>>(p);
+    // no more tiles than SMs: one tile per CTA; where the SMs also suffice for every output chunk of every tile, a
+    // CTA takes one of those
+    p.split = p.n_tiles * p.out_chunks <= sms;
+    if (p.n_tiles <= sms)
+        fused::mlp_forward_kernel<1><<<p.split ? p.n_tiles * p.out_chunks : p.n_tiles, fused::kThreads, fused::kSmemBytes,
+                                       m->stream>>>(p);
+    else fused::mlp_forward_kernel<2><<<sms, fused::kThreads, fused::kSmemBytes, m->stream>>>(p);
     XM_CUDA(cudaGetLastError());
     return XMC_OK;
 }
