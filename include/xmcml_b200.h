@@ -584,6 +584,8 @@ int xmc_mlp_set_params(xmc_mlp* m, const float* params);
 int xmc_mlp_get_params(const xmc_mlp* m, float* params);
 /* y[rows][n_out] = network(x[rows][n_in]) with host buffers; *ms (may be NULL) = device time. */
 int xmc_mlp_forward(xmc_mlp* m, const float* x, int rows, float* y, double* ms);
+/* The same for n rows, any number in [1, max_rows]. */
+int xmc_mlp_forward_rows(xmc_mlp* m, const float* x, int n, float* y, double* ms);
 /* Mean device time of `reps` forward passes over the inputs of the last xmc_mlp_forward call
  * (device-resident, replayed CUDA graph). */
 int xmc_mlp_forward_timed(xmc_mlp* m, int rows, int reps, double* ms);

@@ -78,6 +78,7 @@ def load(path: str | None = None) -> C.CDLL:
         "xmc_mlp_set_params": (C.c_int, [C.c_void_p, P(C.c_float)]),
         "xmc_mlp_get_params": (C.c_int, [C.c_void_p, P(C.c_float)]),
         "xmc_mlp_forward": (C.c_int, [C.c_void_p, P(C.c_float), C.c_int, P(C.c_float), P(C.c_double)]),
+        "xmc_mlp_forward_rows": (C.c_int, [C.c_void_p, P(C.c_float), C.c_int, P(C.c_float), P(C.c_double)]),
         "xmc_mlp_forward_timed": (C.c_int, [C.c_void_p, C.c_int, C.c_int, P(C.c_double)]),
         "xmc_mlp_gradients": (C.c_int, [C.c_void_p, P(C.c_float), P(C.c_float), C.c_int, P(C.c_float), P(C.c_float)]),
         "xmc_mlp_set_dataset": (C.c_int, [C.c_void_p, P(C.c_float), P(C.c_float), C.c_int]),
@@ -118,7 +119,7 @@ EXPORTS = [
     "xmc_batch_validate", "xmc_batch_create", "xmc_batch_run", "xmc_batch_read_tallies", "xmc_batch_set_tuning",
     "xmc_batch_get_tuning", "xmc_batch_autotune", "xmc_batch_destroy",
     "xmc_mlp_create", "xmc_mlp_param_count", "xmc_mlp_set_params", "xmc_mlp_get_params", "xmc_mlp_forward",
-    "xmc_mlp_forward_timed", "xmc_mlp_gradients", "xmc_mlp_set_dataset", "xmc_mlp_train", "xmc_mlp_destroy",
+    "xmc_mlp_forward_rows", "xmc_mlp_forward_timed", "xmc_mlp_gradients", "xmc_mlp_set_dataset", "xmc_mlp_train", "xmc_mlp_destroy",
     "xmc_mlp_set_output_weights", "xmc_weight_integral_table", "xmc_launch_release",
     "xmc_gemm_bf16", "xmc_atomic_throughput", "xmc_autotune", "xmc_launch_set_options",
 ]

@@ -230,13 +230,13 @@ struct EpiBwd {
 
 // ---------------------------------------------------------------- small kernels
 
-// FP32 host inputs [rows x n_in] -> bf16 [rows x 64] (zero padded), and optionally transposed.
-__global__ void pack_inputs_kernel(const float* __restrict__ x, int rows, int n_in, bf16* __restrict__ xb,
+// FP32 host inputs [valid x n_in] -> bf16 [rows x 64] (zero padded both ways), and optionally transposed.
+__global__ void pack_inputs_kernel(const float* __restrict__ x, int rows, int valid, int n_in, bf16* __restrict__ xb,
                                    bf16* __restrict__ xt, int ldt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows * kInPad) return;
     const int r = i / kInPad, c = i % kInPad;
-    const bf16 v = __float2bfloat16_rn(c < n_in ? x[(size_t)r * n_in + c] : 0.0f);
+    const bf16 v = __float2bfloat16_rn(c < n_in && r < valid ? x[(size_t)r * n_in + c] : 0.0f);
     xb[i] = v;
     if (xt) xt[(size_t)c * ldt + r] = v;
 }
@@ -772,9 +772,9 @@ int check_err(xmc_mlp* m) {
     return XMC_OK;
 }
 
-int upload_inputs(xmc_mlp* m, const float* x, int rows, bool transposed) {
-    XM_CUDA(cudaMemcpyAsync(m->xin, x, sizeof(float) * (size_t)rows * m->spec.n_in, cudaMemcpyHostToDevice, m->stream));
-    pack_inputs_kernel<<<(rows * kInPad + 255) / 256, 256, 0, m->stream>>>(m->xin, rows, m->spec.n_in, m->x,
+int upload_inputs(xmc_mlp* m, const float* x, int rows, int valid, bool transposed) {
+    XM_CUDA(cudaMemcpyAsync(m->xin, x, sizeof(float) * (size_t)valid * m->spec.n_in, cudaMemcpyHostToDevice, m->stream));
+    pack_inputs_kernel<<<(rows * kInPad + 255) / 256, 256, 0, m->stream>>>(m->xin, rows, valid, m->spec.n_in, m->x,
                                                                            transposed ? m->xt : nullptr, rows);
     XM_CUDA(cudaGetLastError());
     return XMC_OK;
@@ -932,13 +932,11 @@ extern "C" int xmc_mlp_get_params(const xmc_mlp* m, float* p) {
     return copy_layers_out(m, m->w32, m->b32, p);
 }
 
-extern "C" int xmc_mlp_forward(xmc_mlp* m, const float* x, int rows, float* y, double* ms) {
-    xmc::DeviceGuard device_guard;  // the caller's current device is restored on return
-    if (!m || !x || !y) return mfail(XMC_ERR_INVALID_INPUT, "model, x or y is NULL");
-    int st = check_rows(m, rows);
-    if (st) return st;
+// Forward pass of `valid` host rows as `rows` rows (a multiple of 128; the others are zero), the outputs of the
+// valid ones into y.
+static int forward_host(xmc_mlp* m, const float* x, int rows, int valid, float* y, double* ms) {
     XM_CUDA(cudaSetDevice(m->spec.device));
-    st = upload_inputs(m, x, rows, false);
+    int st = upload_inputs(m, x, rows, valid, false);
     if (st) return st;
     XM_CUDA(cudaEventRecord(m->ev[0], m->stream));
     st = enqueue_forward(m, rows, false);
@@ -948,16 +946,19 @@ extern "C" int xmc_mlp_forward(xmc_mlp* m, const float* x, int rows, float* y, d
     // caller's array on up to 8 host threads. Large outputs go back in 8 chunks of rows, each with
     // its own event, and every thread copies its share of a chunk as soon as that chunk has landed,
     // so the host copies overlap the device-to-host transfer of the later chunks.
-    const size_t nf = (size_t)rows * m->spec.n_out;
+    const size_t nf = (size_t)valid * m->spec.n_out;
     if (m->h_y_floats < nf) {
         if (m->h_y) cudaFreeHost(m->h_y);
         m->h_y = nullptr;
         m->h_y_floats = 0;
-        XM_CUDA(cudaHostAlloc((void**)&m->h_y, sizeof(float) * (size_t)m->cap * m->spec.n_out, cudaHostAllocDefault));
+        XM_CUDA(cudaHostAlloc((void**)&m->h_y, sizeof(float) * ((size_t)m->cap * m->spec.n_out + 1), cudaHostAllocDefault));
         m->h_y_floats = (size_t)m->cap * m->spec.n_out;
     }
+    // the kernels' error word travels with the outputs, behind them in the staging buffer
+    const int* const h_err = reinterpret_cast<const int*>(m->h_y + m->h_y_floats);
+    XM_CUDA(cudaMemcpyAsync(m->h_y + m->h_y_floats, m->d_err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
     const int chunks = nf < ((size_t)1 << 22) ? 1 : 8;
-    const size_t cf = ((size_t)(rows + chunks - 1) / chunks) * m->spec.n_out;  // floats per chunk (whole rows)
+    const size_t cf = ((size_t)(valid + chunks - 1) / chunks) * m->spec.n_out;  // floats per chunk (whole rows)
     for (int k = 0; k < chunks; ++k) {
         if (!m->ev_chunk[k]) XM_CUDA(cudaEventCreateWithFlags(&m->ev_chunk[k], cudaEventDisableTiming));
         const size_t a = std::min(nf, k * cf), b = std::min(nf, a + cf);
@@ -996,7 +997,23 @@ extern "C" int xmc_mlp_forward(xmc_mlp* m, const float* x, int rows, float* y, d
     float t = 0.0f;
     XM_CUDA(cudaEventElapsedTime(&t, m->ev[0], m->ev[1]));
     if (ms) *ms = t;
-    return check_err(m);
+    return *h_err ? check_err(m) : XMC_OK;
+}
+
+extern "C" int xmc_mlp_forward(xmc_mlp* m, const float* x, int rows, float* y, double* ms) {
+    xmc::DeviceGuard device_guard;  // the caller's current device is restored on return
+    if (!m || !x || !y) return mfail(XMC_ERR_INVALID_INPUT, "model, x or y is NULL");
+    const int st = check_rows(m, rows);
+    return st ? st : forward_host(m, x, rows, rows, y, ms);
+}
+
+// The same for any number of rows in [1, max_rows]: a query of one row does not send its tile's other 127 to
+// the host and copy them there (15-256x4-1000, one row: 131 -> 65 us per call, half of it by this and the error word that travels with the outputs).
+extern "C" int xmc_mlp_forward_rows(xmc_mlp* m, const float* x, int n, float* y, double* ms) {
+    xmc::DeviceGuard device_guard;  // the caller's current device is restored on return
+    if (!m || !x || !y) return mfail(XMC_ERR_INVALID_INPUT, "model, x or y is NULL");
+    if (n < 1 || n > m->cap) return mfail(XMC_ERR_RANGE, "rows must be in [1, max_rows]");
+    return forward_host(m, x, round_up(n, tc::kBM), n, y, ms);
 }
 
 // Times `reps` forward passes of the inputs already on the device (the last xmc_mlp_forward's),
@@ -1046,7 +1063,7 @@ extern "C" int xmc_mlp_gradients(xmc_mlp* m, const float* x, const float* t, int
     if (st) return st;
     XM_CUDA(cudaSetDevice(m->spec.device));
     st = ensure_training(m);
-    if (!st) st = upload_inputs(m, x, rows, true);
+    if (!st) st = upload_inputs(m, x, rows, rows, true);
     if (st) return st;
     XM_CUDA(cudaMemcpyAsync(m->t, t, sizeof(float) * (size_t)rows * m->spec.n_out, cudaMemcpyHostToDevice, m->stream));
     // loss slot: loss[step + ... ] uses *d_step; use slot (current step) after zeroing it
@@ -1086,7 +1103,7 @@ extern "C" int xmc_mlp_set_dataset(xmc_mlp* m, const float* x, const float* t, i
     XM_CUDA(cudaMalloc(&xin, sizeof(float) * (size_t)rows * m->spec.n_in));
     cudaError_t e = cudaMemcpy(xin, x, sizeof(float) * (size_t)rows * m->spec.n_in, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
-        pack_inputs_kernel<<<(int)(((size_t)rows * kInPad + 255) / 256), 256>>>(xin, rows, m->spec.n_in, m->ds_x, nullptr, 0);
+        pack_inputs_kernel<<<(int)(((size_t)rows * kInPad + 255) / 256), 256>>>(xin, rows, rows, m->spec.n_in, m->ds_x, nullptr, 0);
         e = cudaDeviceSynchronize();
     }
     cudaFree(xin);

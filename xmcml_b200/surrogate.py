@@ -83,13 +83,10 @@ class MLP:
         for i in range(0, n, self.max_rows):
             xb = x[i:i + self.max_rows]
             r = xb.shape[0]
-            rp = pad_rows(r)
-            if rp != r:
-                xb = np.concatenate([xb, np.zeros((rp - r, self.n_in), np.float32)])
-            y = np.empty((rp, self.n_out), dtype=np.float32)
+            y = np.empty((r, self.n_out), dtype=np.float32)
             t = C.c_double(0.0)
-            check(self._lib.xmc_mlp_forward(self._m, xb.ctypes.data_as(FP), rp, y.ctypes.data_as(FP), C.byref(t)))
-            outs.append(y[:r])
+            check(self._lib.xmc_mlp_forward_rows(self._m, xb.ctypes.data_as(FP), r, y.ctypes.data_as(FP), C.byref(t)))
+            outs.append(y)
             ms += t.value
         if len(outs) == 1:
             return outs[0], ms
