@@ -96,3 +96,18 @@ def test_step_budget_in_both_kernels(tmp_path):
     assert a["n_budget"] > 0
     for k in LEDGER + ["n_budget"]:
         assert a[k] == sum(x[k] for x in b), k
+
+
+def test_contexts_of_different_shared_memory_run_in_turn(tmp_path):
+    """A context that stages much in shared memory still runs, through either kernel, after one was created that
+    stages little."""
+    big = api.Model(*scenes.height_field_tissue(grid=97, n_rings=20, time_bins=5).write(str(tmp_path), "big"))
+    small = api.Model(*scenes.planar(n_rings=2).write(str(tmp_path), "small"))
+    a = api.Transport(big)
+    first = [a.run(n, seed=3)["absorbed_fx"] for n in (500, 90_000)]
+    b = api.Transport(small)
+    b.run(500)
+    assert [a.run(n, seed=3)["absorbed_fx"] for n in (500, 90_000)] == first
+    b.run(90_000)
+    a.close()
+    b.close()

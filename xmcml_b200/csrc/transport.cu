@@ -619,10 +619,22 @@ cudaError_t enqueue_transport(Context* ctx) {
     return log ? enqueue_variant<false, true>(ctx) : enqueue_variant<false, false>(ctx);
 }
 
+// Lets `kernel` take all the dynamic shared memory that a block may have. The limit belongs to the function, not
+// to a context: set to one context's need, it would refuse the launches of another that needs more.
+template <class F>
+static cudaError_t allow_full_smem(F kernel) {
+    int device = 0, optin = 0;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess || fa.maxDynamicSharedSizeBytes >= optin - (int)fa.sharedSizeBytes) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+}
+
 template <bool kBias, bool kLog>
 static cudaError_t tail_occupancy_of(size_t smem, int* blocks_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(transport_tail_kernel<kBias, kLog>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    const cudaError_t e = allow_full_smem(transport_tail_kernel<kBias, kLog>);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, transport_tail_kernel<kBias, kLog>, kTailThreads, smem);
 }
@@ -646,7 +658,7 @@ static cudaError_t occupancy_of(int block, size_t smem, int* blocks_per_sm) {
         *blocks_per_sm = 0;
         return cudaSuccess;
     }
-    e = cudaFuncSetAttribute(transport_kernel<kBias, kLog>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_full_smem(transport_kernel<kBias, kLog>);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, transport_kernel<kBias, kLog>, block, smem);
 }
