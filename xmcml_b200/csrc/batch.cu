@@ -707,6 +707,7 @@ struct xmc_batch {
     // device
     unsigned char* d_misc = nullptr;  // [0,16) header, [64,72) dispenser, [72,76) status, [80,88) tail counts
     BatchTail* d_tail = nullptr;      // photons handed over to the tail kernel
+    size_t tail_cap = 0;
     int tail_grid = 0;
     BInst* d_inst = nullptr;
     float4* d_layers = nullptr;
@@ -852,6 +853,15 @@ int apply_tuning(xmc_batch* b, const xmc_batch_tuning& t) {
     int st = occupancy(t.tally_scheme, t.block_size, &occ);
     if (st) return st;
     const int bps = t.blocks_per_sm > 0 ? std::min(t.blocks_per_sm, occ) : occ;
+    // the tail list holds what the grid's threads may hand over
+    const size_t threads = (size_t)b->sms * bps * t.block_size;
+    if (threads > b->tail_cap) {
+        BatchTail* list = nullptr;
+        XB_CUDA(cudaMalloc(&list, sizeof(BatchTail) * threads));
+        cudaFree(b->d_tail);
+        b->d_tail = list;
+        b->tail_cap = threads;
+    }
     for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
     b->graphs.clear();
     b->tuning = t;
@@ -998,13 +1008,9 @@ extern "C" int xmc_batch_create(const xmc_batch_spec* spec, xmc_batch** out) {
     XB_TRY(cudaMalloc(&b->d_ring, sizeof(unsigned long long) * 3 * R * cap));
     XB_TRY(cudaMalloc(&b->d_tbin, sizeof(unsigned long long) * 3 * R * T * cap));
     XB_TRY(cudaMalloc(&b->d_ledger, sizeof(unsigned long long) * XMC_BATCH_LEDGER * cap));
-    // the tail list holds what every warp that an SM can keep resident may hand over
-    int tail_occ = 0, warps = 0;
+    int tail_occ = 0;
     XB_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tail_occ, batch_tail_kernel, kBatchTailThreads, 0));
-    XB_TRY(cudaDeviceGetAttribute(&warps, cudaDevAttrMaxThreadsPerMultiProcessor, s.device));
-    warps /= 32;
     b->tail_grid = b->sms * std::max(1, tail_occ);
-    XB_TRY(cudaMalloc(&b->d_tail, sizeof(BatchTail) * 32 * (size_t)b->sms * warps));
     XB_TRY(cudaMalloc(&b->d_ring_f, sizeof(double) * R * cap));
     XB_TRY(cudaMalloc(&b->d_tbin_f, sizeof(double) * R * T * cap));
     XB_TRY(cudaMallocHost(&b->h_hdr, 16));

@@ -509,7 +509,7 @@ static int create_from_image(const HostImage& img, Context** out) {
     CK(up(&c->d_cell_entries, img.grid.entries.data(), sizeof(float4) * img.grid.entries.size()));
     CK(up(&c->d_big, img.grid.big.data(), sizeof(float4) * img.grid.big.size()));
     CK(up(&c->d_cell_runs, img.grid.cell_runs.data(), sizeof(uint32_t) * img.grid.cell_runs.size()));
-    CK(up(&c->d_clear, img.clear.data(), img.clear.size()));
+    if (!img.clear.empty()) CK(up(&c->d_clear, img.clear.data(), img.clear.size()));
     if (img.kp.use_bias) {
         CK(up(&c->d_wtab, img.wtab.data(), sizeof(float) * img.wtab.size()));
         c->h2d_bytes += sizeof(float) * img.wtab.size();

@@ -151,8 +151,9 @@ constexpr int kMaxZSlabs = 24;
 // bounds only the others count, by their merged z-intervals.
 constexpr int kMaxClearance = 15;
 constexpr int kClearanceRim = 4;
-constexpr int kClearanceAxis = 256;  // voxels along one axis, without the rim
-constexpr int kClearanceVoxels = 1 << 18;  // 2^15: 3 % slower on the ellipsoid, 2^21: 2 % faster and 8 times the build
+constexpr int kClearanceAxis = 128;  // voxels along one axis, without the rim
+constexpr int kClearanceVoxels = 1 << 16;  // the ellipsoid: 2^15 87 ps per step, 2^18 84, 2^21 82; but 2^18 and 256 along an
+                                           // axis took 60 ms of a height field's context
 
 // Everything the kernel reads, by value (kernel parameter space).
 struct KParams {
