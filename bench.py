@@ -493,7 +493,7 @@ def measure_batch(args, rank, world, local, dist, torch, barrier, n_steps, n_war
             "e2e": {"value": world * n_steps * total / wall_s, "unit": UNIT,
                     "h2d_bytes_per_step": K * (32 + 5 * 48), "d2h_bytes_per_step": K * (R * T * 8 + R * 8 + 16 * 8) + 4,
                     "via": "xmc_batch_run with host instance table and host result arrays"},
-            "gpu_launches": 2 * n_steps, "roofline": rl, "cpu_baseline": cpu,
+            "gpu_launches": 3 * n_steps, "roofline": rl, "cpu_baseline": cpu,
             "walk": {"steps_per_photon": steps / total}}
     if cpu and cpu.get("value"):
         cpu["gpu_value_over_cpu"] = value / cpu["value"]
@@ -557,7 +557,7 @@ def main():
             line["surrogate"] = {"metric": "surrogate evals/s", "value": None, "error": str(e)}
     line["gpu_launches"] = line["gpu_launches"] + sum(v["gpu_launches"] for v in extra.values()) + (
         line["roulette_variant"]["gpu_launches"] if "roulette_variant" in line else 0)
-    line["gpu_launches_note"] = ("transport kernel launches (run pass + trajectory replay pass per call) of the timed "
+    line["gpu_launches_note"] = ("transport and tail kernel launches (and the trajectory replay pass of a call) of the timed "
                                  "steps of the headline, the roulette variant and the extra workloads, and the batched "
                                  "sweep's kernel and reduction per timed step")
     if rank == 0:
@@ -605,7 +605,7 @@ def measure_transport(args, workload, N, steps, warmup, e2e_steps, rank, world, 
     value = world * steps * N / (dev_ms / 1e3)
     last = leds[-1]
     traj_adds = int(t.maps()["trajectory"].sum()) if maps else 0  # one atomic add per counted crossing
-    launches = sum(1 + (1 if l["n_trajectory_replayed"] > 0 else 0) for l in leds)
+    launches = sum(2 + (1 if l["n_trajectory_replayed"] > 0 else 0) for l in leds)
     shape = {"block": tuned.block_size or 256, "photons_per_claim": tuned.photons_per_chunk,
              "queries": "lane by lane" if tuned.flags & S.XMC_LANE_QUERIES else "warp-cooperative",
              "query_batch": max(1, tuned.query_batch), "grid_cell_tris": tuned.grid_cell_tris or 2,
