@@ -76,9 +76,11 @@ class MLP:
             check(self._lib.xmc_mlp_set_output_weights(self._m, w.ctypes.data_as(FP)))
 
     def forward(self, x: np.ndarray) -> Tuple[np.ndarray, float]:
-        """(outputs [n, n_out] float32, device ms); rows padded to a multiple of 128 internally."""
+        """(outputs [n, n_out] float32, device ms) for x [n, n_in]."""
         x = _f32(x)
         n = x.shape[0]
+        if n and (x.ndim != 2 or x.shape[1] != self.n_in):  # the library reads n x n_in floats from a pointer
+            raise ValueError(f"forward takes an array [n, {self.n_in}], not {list(x.shape)}")
         outs, ms = [], 0.0
         for i in range(0, n, self.max_rows):
             xb = x[i:i + self.max_rows]
