@@ -1,5 +1,5 @@
 """Arrays of the wrong shape are refused before a pointer to them reaches the library, which reads rows x n_in
-floats from it. The library is a stand-in that notes its calls: no GPU needed."""
+(rows x n_out for targets) floats from it. The library is a stand-in that notes its calls: no GPU needed."""
 import ctypes as C
 
 import numpy as np
@@ -18,7 +18,12 @@ class _Library:
         self.rows.append(rows)
         return 0
 
+    def _note_two(self, handle, x, t, rows, *_):
+        self.rows.append(rows)
+        return 0
+
     xmc_mlp_forward_rows = _note
+    xmc_mlp_gradients = xmc_mlp_set_dataset = _note_two
 
     def xmc_mlp_destroy(self, handle):
         return 0
@@ -54,3 +59,21 @@ def test_ensemble_mean_refuses_a_flat_query():
     with pytest.raises(ValueError):
         s.mean_log10(np.zeros(N_IN))
     assert s.members[0]._lib.rows == []
+
+
+@pytest.mark.parametrize("call", ["gradients", "set_dataset"])
+@pytest.mark.parametrize("x,t", [((128, N_IN - 1), (128, N_OUT)), ((128, N_IN + 1), (128, N_OUT)), ((128, N_IN), (128, N_OUT - 1)),
+                                 ((128, N_IN), (127, N_OUT)), ((128 * N_IN,), (128, N_OUT)), ((128, N_IN), (128,))])
+def test_training_arrays_of_other_shapes_are_refused(call, x, t):
+    m = _net()
+    with pytest.raises(ValueError):
+        getattr(m, call)(np.zeros(x, np.float32), np.zeros(t, np.float32))
+    assert m._lib.rows == []
+
+
+@pytest.mark.parametrize("call", ["gradients", "set_dataset"])
+@pytest.mark.parametrize("t", [(128, N_OUT), (128, 4, 5), (200, N_OUT)])
+def test_training_takes_targets_laid_out_as_rings_and_bins(call, t):
+    m = _net()
+    getattr(m, call)(np.zeros((128, N_IN), np.float32), np.zeros(t, np.float32))
+    assert m._lib.rows == [128]

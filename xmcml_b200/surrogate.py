@@ -99,8 +99,17 @@ class MLP:
         check(self._lib.xmc_mlp_forward_timed(self._m, rows, reps, C.byref(t)))
         return t.value
 
-    def gradients(self, x: np.ndarray, t: np.ndarray) -> Tuple[np.ndarray, float]:
+    def _training_rows(self, x: np.ndarray, t: np.ndarray) -> Tuple[np.ndarray, np.ndarray]:
+        """x and t as float32 arrays of at least len(x) rows of n_in and n_out values (a row of any shape, so that
+        targets may be laid out as rings x time bins): the library reads that many from two pointers."""
         x, t = _f32(x), _f32(t)
+        if x.size != len(x) * self.n_in or t.size != len(t) * self.n_out or len(t) < len(x):
+            raise ValueError(f"training takes rows of {self.n_in} inputs and as many of {self.n_out} targets, "
+                             f"not {list(x.shape)} and {list(t.shape)}")
+        return x, t
+
+    def gradients(self, x: np.ndarray, t: np.ndarray) -> Tuple[np.ndarray, float]:
+        x, t = self._training_rows(x, t)
         g = np.zeros(self.n_params, dtype=np.float32)
         loss = C.c_float(0.0)
         check(self._lib.xmc_mlp_gradients(self._m, x.ctypes.data_as(FP), t.ctypes.data_as(FP), x.shape[0],
@@ -108,7 +117,7 @@ class MLP:
         return g, loss.value
 
     def set_dataset(self, x: np.ndarray, t: np.ndarray) -> None:
-        x, t = _f32(x), _f32(t)
+        x, t = self._training_rows(x, t)
         self._ds = (x, t)
         check(self._lib.xmc_mlp_set_dataset(self._m, x.ctypes.data_as(FP), t.ctypes.data_as(FP), x.shape[0]))
 
