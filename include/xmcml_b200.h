@@ -448,6 +448,10 @@ int xmc_layout_offsets(int64_t* out, int max_count);
 int xmc_debug_nearest(const InputInfo* input, int n_rays, const float* rays, float tmin, float tmax,
                       float* t_out, int* surf_out, float* normal_out, int flags);
 
+/* The batch kernels' rule compiled for the host: a step that ends between *zlo and *zhi of a layer with planes
+ * at z_top and z_bot and mean free path inv_mut has reached neither plane. Used by the test suites. */
+void xmc_debug_free_depths(float z_top, float z_bot, float inv_mut, float* zlo, float* zhi);
+
 /* Run the photon kernel's device-side self test: `n` Philox blocks for the given key written to
  * out[4*n] (device path), for comparing with xmc_philox4x32_10. */
 int xmc_device_philox(uint64_t seed, uint64_t photon_id, uint32_t n, uint32_t* out);
