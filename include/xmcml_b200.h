@@ -452,6 +452,10 @@ int xmc_debug_nearest(const InputInfo* input, int n_rays, const float* rays, flo
  * at z_top and z_bot and mean free path inv_mut has reached neither plane. Used by the test suites. */
 void xmc_debug_free_depths(float z_top, float z_bot, float inv_mut, float* zlo, float* zhi);
 
+/* Counts since the library was loaded, into out[0..max_count); returns how many there are. [0] transport and
+ * batch runs that a tail kernel walked whole. Used by the test suites. */
+int xmc_debug_counts(uint64_t* out, int max_count);
+
 /* Run the photon kernel's device-side self test: `n` Philox blocks for the given key written to
  * out[4*n] (device path), for comparing with xmc_philox4x32_10. */
 int xmc_device_philox(uint64_t seed, uint64_t photon_id, uint32_t n, uint32_t* out);

@@ -53,7 +53,7 @@ constexpr int kLayerF4 = 3;
 struct BatchParams {
     const BInst* inst;
     const float4* layers;
-    const unsigned long long* hdr;  // [0] instances, [1] photons of all instances
+    const unsigned long long* hdr;  // [0] instances, [1] photons of all instances, [2] 1: the tail kernel walks them all
     int stride;                     // n_layers + 2
     int n_layers;
     int n_rings, n_time;
@@ -67,7 +67,6 @@ struct BatchParams {
     int* status;
     struct BatchTail* tail;      // photons that the last warps hand over to the tail kernel
     unsigned* tail_count;        // photons listed, then the tail kernel's dispenser of them
-    unsigned long long direct_max;  // runs of at most this many photons go to the tail kernel whole
     unsigned long long* ring;    // [instance][ring][3]
     unsigned long long* tbin;    // [instance][ring][time][3]
     unsigned long long* ledger;  // [instance][XMC_BATCH_LEDGER]
@@ -221,7 +220,7 @@ __global__ void __launch_bounds__(256, 3) batch_kernel(const BatchParams P) {
     const unsigned lt_mask = (1u << lane) - 1u;
     const int n_inst = (int)P.hdr[0];
     const unsigned long long total = P.hdr[1];
-    if (total <= P.direct_max) return;
+    if (P.hdr[2]) return;
 
     unsigned long long cbeg = 0, cend = 0;  // warp-uniform chunk of global photon indices
     bool exhausted = false, alive = false;
@@ -425,7 +424,7 @@ __global__ void __launch_bounds__(256, 3) batch_kernel(const BatchParams P) {
 __global__ void __launch_bounds__(kBatchTailThreads) batch_tail_kernel(const BatchParams P) {
     constexpr int G = kBatchTailGroup, D = G * kBatchTailDraws;
     const unsigned long long total = P.hdr[1];
-    const bool direct = total <= P.direct_max;  // from the id dispenser, else from the list
+    const bool direct = P.hdr[2] != 0;  // from the id dispenser, else from the list
     const unsigned n_listed = direct ? 0u : P.tail_count[0];
     if (!direct && blockIdx.x >= n_listed) return;  // nothing for this block
     // the groups' draws: {step length, cos theta, sin theta, sin azimuth}, cos azimuth
@@ -715,10 +714,11 @@ struct xmc_batch {
     xmc_batch_tuning tuning{256, 0, 64, 1, 0.0};
     int grid = 0, block = 0;
     // device
-    unsigned char* d_misc = nullptr;  // [0,16) header, [64,72) dispenser, [72,76) status, [80,88) tail counts
+    unsigned char* d_misc = nullptr;  // [0,24) header, [64,72) dispenser, [72,76) status, [80,88) tail counts
     BatchTail* d_tail = nullptr;      // photons handed over to the tail kernel
     size_t tail_cap = 0;
     int tail_grid = 0;
+    bool tail_takes_small_runs = true;  // false while the shape of the batch kernel is tuned
     BInst* d_inst = nullptr;
     float4* d_layers = nullptr;
     unsigned long long *d_ring = nullptr, *d_tbin = nullptr, *d_ledger = nullptr;
@@ -809,6 +809,8 @@ void pack(xmc_batch* b, const xmc_batch_instance* inst, int n) {
     }
     b->h_hdr[0] = (unsigned long long)n;
     b->h_hdr[1] = first;
+    // fewer photons than the grid has threads: every warp would be thin from the start
+    b->h_hdr[2] = b->tail_takes_small_runs && first <= (unsigned long long)b->grid * b->block;
 }
 
 BatchParams params(const xmc_batch* b) {
@@ -836,7 +838,6 @@ BatchParams params(const xmc_batch* b) {
     P.counter = reinterpret_cast<unsigned long long*>(b->d_misc + 64);
     P.status = reinterpret_cast<int*>(b->d_misc + 72);
     P.tail = b->d_tail;
-    P.direct_max = (unsigned long long)b->grid * b->block;
     P.tail_count = reinterpret_cast<unsigned*>(b->d_misc + 80);
     P.ring = b->d_ring;
     P.tbin = b->d_tbin;
@@ -886,7 +887,7 @@ int enqueue(xmc_batch* b, int n, bool capturing) {
     const xmc_batch_spec& s = b->spec;
     const size_t R = (size_t)s.n_rings, T = (size_t)s.n_time;
     cudaStream_t st = b->stream;
-    XB_CUDA(cudaMemcpyAsync(b->d_misc, b->h_hdr, 16, cudaMemcpyHostToDevice, st));
+    XB_CUDA(cudaMemcpyAsync(b->d_misc, b->h_hdr, 24, cudaMemcpyHostToDevice, st));
     XB_CUDA(cudaMemcpyAsync(b->d_inst, b->h_inst, sizeof(BInst) * n, cudaMemcpyHostToDevice, st));
     XB_CUDA(cudaMemcpyAsync(b->d_layers, b->h_layers, sizeof(float4) * kLayerF4 * b->stride * (size_t)n,
                             cudaMemcpyHostToDevice, st));
@@ -946,6 +947,7 @@ int graph_for(xmc_batch* b, int n, cudaGraphExec_t* out) {
 
 // One run of n >= 1 packed instances; waits for it.
 int run_packed(xmc_batch* b, int n, bool use_graph, double* kernel_ms) {
+    if (b->h_hdr[2]) ++g_debug_counts.whole_in_tail;
     if (use_graph) {
         cudaGraphExec_t ex = nullptr;
         int st = graph_for(b, n, &ex);
@@ -1023,7 +1025,7 @@ extern "C" int xmc_batch_create(const xmc_batch_spec* spec, xmc_batch** out) {
     b->tail_grid = b->sms * std::max(1, tail_occ);
     XB_TRY(cudaMalloc(&b->d_ring_f, sizeof(double) * R * cap));
     XB_TRY(cudaMalloc(&b->d_tbin_f, sizeof(double) * R * T * cap));
-    XB_TRY(cudaMallocHost(&b->h_hdr, 16));
+    XB_TRY(cudaMallocHost(&b->h_hdr, 24));
     XB_TRY(cudaMallocHost(&b->h_inst, sizeof(BInst) * cap));
     XB_TRY(cudaMallocHost(&b->h_layers, sizeof(float4) * kLayerF4 * b->stride * cap));
     XB_TRY(cudaMallocHost(&b->h_ring_f, sizeof(double) * R * cap));
@@ -1121,7 +1123,11 @@ extern "C" int xmc_batch_autotune(xmc_batch* b, const xmc_batch_instance* sample
     std::vector<xmc_batch_instance> capped(sample, sample + n);
     for (auto& I : capped)
         if (photons_cap > 0) I.photons = std::min<uint64_t>(I.photons, photons_cap);
+    // every sample goes through the kernel whose shape is chosen: one that the tail kernel walks whole would time
+    // that, and noise would choose
+    b->tail_takes_small_runs = false;
     pack(b, capped.data(), n);
+    b->tail_takes_small_runs = true;
     const xmc_batch_tuning keep = b->tuning;
     xmc_batch_tuning win{};
     win.ms = INFINITY;

@@ -20,6 +20,8 @@ static thread_local std::string g_last_error;
 
 void set_error(const std::string& msg) { g_last_error = msg; }
 
+DebugCounts g_debug_counts;
+
 static int fail(int status, const std::string& msg) {
     set_error(msg);
     return status;
@@ -963,6 +965,8 @@ static int time_shape(const HostImage& img, uint64_t n, uint64_t seed, double* m
     Context* c = nullptr;
     int st = create_from_image(img, &c);
     if (st) return st;
+    // a sample that the tail kernel walks whole would time that instead of the shape
+    c->tail_takes_small_runs = false;
     xmc_ledger led;
     st = run(c, seed, 0, std::max<uint64_t>(n / 4, 1), nullptr, &led);
     if (!st || st == XMC_ERR_BUDGET) st = run(c, seed + 1, 0, n, nullptr, &led);
@@ -1210,6 +1214,13 @@ int xmc_launch_omp(InputInfo* input, OutputInfo* output, MCG59* rng, int numThre
     // (the next backup portion) uses a fresh key
     rng[0].value = (rng[0].value * rng[0].offset) & 576460752303423487ULL;
     return st;
+}
+
+int xmc_debug_counts(uint64_t* out, int max_count) {
+    const uint64_t v[] = {g_debug_counts.whole_in_tail};
+    const int n = (int)(sizeof(v) / sizeof(v[0]));
+    for (int i = 0; out && i < std::min(n, max_count); ++i) out[i] = v[i];
+    return n;
 }
 
 double xmc_specular_reflectance(const LayerInfo* layer) { return specular(layer); }

@@ -1,6 +1,7 @@
 // Internal declarations shared by the host C++ files and the CUDA transport kernel.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <thread>
@@ -263,6 +264,7 @@ struct Context {
     int block = 256, blocks_per_sm = 0, num_sms = 0, grid = 0;
     int tail_grid = 0;        // blocks of the tail kernel (0: not used)
     size_t tail_smem = 0;
+    bool tail_takes_small_runs = true;  // false while the shape of the transport kernel is tuned
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     // device buffers
@@ -380,6 +382,12 @@ cudaError_t tail_occupancy(const KParams& kp, size_t* smem, int* blocks_per_sm, 
 cudaError_t device_philox(uint32_t key0, uint32_t key1, uint64_t pid, uint32_t n, uint32_t* host_out);
 
 void set_error(const std::string& msg);
+
+// What the test suites cannot see in results (xmc_debug_counts).
+struct DebugCounts {
+    std::atomic<uint64_t> whole_in_tail{0};  // runs that a tail kernel walked whole
+};
+extern DebugCounts g_debug_counts;  // capi.cpp
 
 // Keeps the caller's current CUDA device across an entry point: the device current on entry is
 // made current again when the guard goes out of scope (every return path), so an entry point that
