@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <iterator>
 #include <mutex>
 #include <new>
 #include <string>
@@ -976,22 +977,51 @@ static int time_shape(const HostImage& img, uint64_t n, uint64_t seed, double* m
     return XMC_OK;
 }
 
+// Triangles per cell of the xy grids that xmc_autotune builds.
+static const int kTuneDensities[] = {2, 8, 16, 32};
+
+// The launch shapes that it times on one of them.
+static std::vector<xmc_options> launch_shapes(const xmc_options& base) {
+    const int blocks[] = {256, 512};
+    const int chunks[] = {32, 64};
+    // lanes that wait for a general step, in either query scheme. Not 1 (1e6 photons, ms at 1 / 8 / 12 / 16 lanes:
+    // height field 70 / 41 / 39 / 41, lane by lane 105 / 66 / 62 / 61; ellipsoid 71 / 50 / 48 / 50, 94 / 71 / 68 / 70;
+    // glass cover 30 / 18 / 16 / 15, 34 / 21 / 18 / 16)
+    const int batches[] = {8, 12, 16};
+    std::vector<xmc_options> shapes;
+    for (int coop = 1; coop >= 0; --coop)
+        for (int b : blocks)
+            for (int ch : chunks)
+                for (int qb : batches) {
+                    xmc_options c = base;
+                    c.block_size = b;
+                    c.blocks_per_sm = 0;
+                    c.photons_per_chunk = ch;
+                    c.query_batch = qb;
+                    c.flags = coop ? (c.flags & ~XMC_LANE_QUERIES) : (c.flags | XMC_LANE_QUERIES);
+                    shapes.push_back(c);
+                }
+    return shapes;
+}
+
+int xmc_debug_launch_shapes(const xmc_options* base, xmc_options* out, int max_count) {
+    const std::vector<xmc_options> shapes = launch_shapes(*base);
+    for (int i = 0; out && i < std::min((int)shapes.size(), max_count); ++i) out[i] = shapes[i];
+    return (int)shapes.size();
+}
+
 int xmc_autotune(const InputInfo* input, const xmc_options* base, uint64_t sample_photons, xmc_options* best,
                  double* best_ms) {
     if (!input || !best) return fail(XMC_ERR_INVALID_INPUT, "xmc_autotune: NULL argument");
     set_error("");
     DeviceGuard device_guard;
     const uint64_t n = sample_photons ? sample_photons : 1000000ull;
-    const int densities[] = {2, 8, 16, 32};
-    const int n_dens = (int)(sizeof(densities) / sizeof(densities[0]));
-    const int blocks[] = {256, 512};
-    const int chunks[] = {32, 64};
-    const int batches[] = {1, 8, 12, 16};
     struct Cand {
         xmc_options opt;
         double ms;
     };
     std::vector<Cand> cands;
+    const int n_dens = (int)std::size(kTuneDensities);
     std::vector<HostImage> images(n_dens);
     std::string last_err;
     for (int di = 0; di < n_dens; ++di) {
@@ -1000,31 +1030,16 @@ int xmc_autotune(const InputInfo* input, const xmc_options* base, uint64_t sampl
         xmc_default_options(&o);
         if (base && base->struct_size) std::memcpy(&o, base, std::min((size_t)base->struct_size, sizeof(o)));
         o.struct_size = sizeof(o);
-        o.grid_cell_tris = densities[di];
+        o.grid_cell_tris = kTuneDensities[di];
         HostImage& img = images[di];
         int st = full_image(input, &o, &img);
         if (st) return st;
-        for (int coop = 1; coop >= 0; --coop) {
-            for (int b : blocks) {
-                for (int ch : chunks) {
-                    for (int qb : batches) {
-                        if (!coop && qb > 1) continue;  // query batches apply to the cooperative scheme only
-                        xmc_options c = img.opt;
-                        c.block_size = b;
-                        c.blocks_per_sm = 0;
-                        c.photons_per_chunk = ch;
-                        c.query_batch = qb;
-                        c.flags = coop ? (c.flags & ~XMC_LANE_QUERIES) : (c.flags | XMC_LANE_QUERIES);
-                        cands.push_back({c, INFINITY});
-                    }
-                }
-            }
-        }
+        for (const xmc_options& c : launch_shapes(img.opt)) cands.push_back({c, INFINITY});
     }
     // launch-shape fields only: the tally arithmetic stays the same
     auto shaped = [&](const xmc_options& c) {
         int di = 0;
-        while (di + 1 < n_dens && densities[di] != c.grid_cell_tris) ++di;
+        while (di + 1 < n_dens && kTuneDensities[di] != c.grid_cell_tris) ++di;
         HostImage img = images[di];
         img.opt = c;
         img.kp.flags = c.flags;

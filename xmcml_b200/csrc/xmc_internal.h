@@ -178,8 +178,8 @@ struct KParams {
     int grid_nx, grid_ny;
     int coop_query;           // 1: grid queries run warp-cooperatively (WarpQuery scratch per warp in
                               // shared memory); 0: each lane walks its own cells
-    int query_batch;          // cooperative: a warp runs its query round once this many lanes wait (or
-                              // every live lane waits)
+    int query_batch;          // a warp takes its lanes' general steps together once this many lanes wait for one
+                              // (or every live lane does), in either query scheme
     // clearance grid (clear_n[0] == 0: none)
     const uint8_t* clear;
     float clear_o[3], clear_i[3];     // origin, 1 / voxel size
