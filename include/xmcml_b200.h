@@ -453,7 +453,7 @@ int xmc_debug_nearest(const InputInfo* input, int n_rays, const float* rays, flo
 void xmc_debug_free_depths(float z_top, float z_bot, float inv_mut, float* zlo, float* zhi);
 
 /* Counts since the library was loaded, into out[0..max_count); returns how many there are. [0] transport and
- * batch runs that a tail kernel walked whole. Used by the test suites. */
+ * batch runs that a tail kernel walked whole; [1] clearance grids built. Used by the test suites. */
 int xmc_debug_counts(uint64_t* out, int max_count);
 
 /* The launch shapes that xmc_autotune times on each grid density, made from `base`, into out[0..max_count);

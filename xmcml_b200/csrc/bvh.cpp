@@ -467,6 +467,7 @@ void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std
         for (int c = 0; c < 3; ++c) big.tris.push_back(v[c]);
     }
     if (big.n_tris >= g.n_tris) return;  // no others: the z-gaps say all there is
+    ++g_debug_counts.clearance_grids;
     kp->n_zbig = occupied_z_slabs(big, kp->zbig_lo, kp->zbig_hi);
     // padded boxes of the small triangles, and their bounds
     auto box = [&](int t, float* lo, float* hi) {

@@ -147,7 +147,7 @@ static int validate(const InputInfo* in, const xmc_options& opt) {
     return XMC_OK;
 }
 
-int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img) {
+int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img, bool clearance) {
     xmc_options opt;
     xmc_default_options(&opt);
     if (opt_in && opt_in->struct_size) {
@@ -311,7 +311,7 @@ int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img
         else build_xy_grid(geom, &img->grid, opt.grid_cell_tris > 0 ? opt.grid_cell_tris : 12);
     });
     kp.n_zocc = n_zocc;
-    build_clearance(geom, img->grid, &kp, &img->clear);
+    if (clearance) build_clearance(geom, img->grid, &kp, &img->clear);
     kp.grid_x0 = img->grid.x0;
     kp.grid_y0 = img->grid.y0;
     kp.grid_icx = img->grid.icx;
@@ -1232,7 +1232,7 @@ int xmc_launch_omp(InputInfo* input, OutputInfo* output, MCG59* rng, int numThre
 }
 
 int xmc_debug_counts(uint64_t* out, int max_count) {
-    const uint64_t v[] = {g_debug_counts.whole_in_tail};
+    const uint64_t v[] = {g_debug_counts.whole_in_tail, g_debug_counts.clearance_grids};
     const int n = (int)(sizeof(v) / sizeof(v[0]));
     for (int i = 0; out && i < std::min(n, max_count); ++i) out[i] = v[i];
     return n;

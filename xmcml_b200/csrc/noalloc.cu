@@ -71,7 +71,9 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     if (opt && opt->struct_size) std::memcpy(&o, opt, std::min((size_t)opt->struct_size, sizeof(o)));
     o.flags &= ~XMC_GPU_BVH;
     o.flags |= XMC_LANE_QUERIES;  // the cooperative query's entry records would need more scratch
-    int st = prepare_image(input, &o, &img);
+    // no clearance grid: it is not staged, and each call would build it again (height field of 2 x 64 x 64 cells:
+    // 13.6 -> 11.1 ms per call of 10 photons)
+    int st = prepare_image(input, &o, &img, false);
     if (st) return st;
     if (img.kp.use_bias) {
         set_error("xmc_run_noalloc: biasing needs weight tables this entry point does not stage");
@@ -136,7 +138,6 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     kp.counter = reinterpret_cast<unsigned long long*>(scratch);
     kp.status = reinterpret_cast<int*>(scratch + sizeof(unsigned long long));
     kp.cancel = nullptr;
-    kp.clear_n[0] = 0;  // the clearance grid is not staged: every segment outside the z-gaps is queried
     kp.absorb = d_absorption;
     kp.det = d_detectors;
     kp.tbin = d_time_bins;

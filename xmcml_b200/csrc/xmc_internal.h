@@ -346,8 +346,9 @@ std::vector<double> distinct_anisotropies(const InputInfo* in);
 int set_weight_tables(const InputInfo* in, const std::vector<double>& gs, const std::vector<double>& tables, int n_elem,
                       HostImage* img);
 
-// capi.cpp: validate `in` and build its host image (options normalised as xmc_create does).
-int prepare_image(const InputInfo* in, const xmc_options* opt, HostImage* img);
+// capi.cpp: validate `in` and build its host image (options normalised as xmc_create does). Without the clearance
+// grid every segment outside the z-gaps is queried.
+int prepare_image(const InputInfo* in, const xmc_options* opt, HostImage* img, bool clearance = true);
 // capi.cpp: fill a ledger from the raw device ledger slots of a run of n photons.
 void fill_ledger(const unsigned long long* raw, uint32_t w0_fx, uint64_t n, xmc_ledger* led);
 
@@ -385,7 +386,8 @@ void set_error(const std::string& msg);
 
 // What the test suites cannot see in results (xmc_debug_counts).
 struct DebugCounts {
-    std::atomic<uint64_t> whole_in_tail{0};  // runs that a tail kernel walked whole
+    std::atomic<uint64_t> whole_in_tail{0};    // runs that a tail kernel walked whole
+    std::atomic<uint64_t> clearance_grids{0};  // clearance grids built
 };
 extern DebugCounts g_debug_counts;  // capi.cpp
 
