@@ -23,6 +23,7 @@
 #include <cstring>
 #include <deque>
 #include <functional>
+#include <memory>
 
 #include "xmc_internal.h"
 
@@ -451,50 +452,66 @@ int occupied_z_slabs(const GeomImage& g, float* lo, float* hi) {
 void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std::vector<uint8_t>* clear) {
     kp->clear_n[0] = kp->clear_n[1] = kp->clear_n[2] = 0;
     clear->clear();
-    // big or horizontal triangles: their z-intervals say enough
-    std::vector<char> is_big((size_t)g.n_tris, 0);
+    // padded boxes of the small triangles, each host thread a range, and their bounds
+    struct Box { float lo[3], hi[3]; };
+    const unsigned parts = std::min(8u, host_parts(g.n_tris));
+    std::vector<char> is_big;
+    std::vector<Box> bounds;
+    std::unique_ptr<Box[]> box;  // first touched by the threads that fill it
     GeomImage big;
-    for (size_t k = 0; k < grid.big.size(); k += 4) {
-        int t;
-        std::memcpy(&t, &grid.big[k].z, sizeof(t));
-        is_big[t] = 1;
+    try {
+        is_big.assign((size_t)g.n_tris, 0);
+        box.reset(new Box[(size_t)g.n_tris]);
+        bounds.assign(parts, Box{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}});
+        // big or horizontal triangles: their z-intervals say enough
+        for (size_t k = 0; k < grid.big.size(); k += 4) {
+            int t;
+            std::memcpy(&t, &grid.big[k].z, sizeof(t));
+            is_big[t] = 1;
+        }
+        const size_t per = ((size_t)g.n_tris + parts - 1) / parts;
+        parallel_parts(parts, [&](unsigned part) {
+            Box all = bounds[part];
+            const size_t t1 = std::min((size_t)g.n_tris, (part + 1) * per);
+            for (size_t t = std::min((size_t)g.n_tris, part * per); t < t1; ++t) {
+                const float4 a = g.tris[3 * t], b = g.tris[3 * t + 1], c = g.tris[3 * t + 2];
+                if (a.z == b.z && a.z == c.z) is_big[t] = 1;
+                if (is_big[t]) continue;
+                const float v[3][3] = {{a.x, b.x, c.x}, {a.y, b.y, c.y}, {a.z, b.z, c.z}};
+                Box& x = box[t];
+                for (int d = 0; d < 3; ++d) {
+                    x.lo[d] = std::min(v[d][0], std::min(v[d][1], v[d][2]));
+                    x.hi[d] = std::max(v[d][0], std::max(v[d][1], v[d][2]));
+                    const float pad = 2e-5f * std::max(1.0f, std::max(std::fabs(x.lo[d]), std::fabs(x.hi[d])));
+                    x.lo[d] -= pad;
+                    x.hi[d] += pad;
+                    all.lo[d] = std::min(all.lo[d], x.lo[d]);
+                    all.hi[d] = std::max(all.hi[d], x.hi[d]);
+                }
+            }
+            bounds[part] = all;
+        });
+        for (int t = 0; t < g.n_tris; ++t) {
+            if (!is_big[t]) continue;
+            ++big.n_tris;
+            for (int c = 0; c < 3; ++c) big.tris.push_back(g.tris[3 * (size_t)t + c]);
+        }
+        if (big.n_tris >= g.n_tris) return;  // no others: the z-gaps say all there is
+        kp->n_zbig = occupied_z_slabs(big, kp->zbig_lo, kp->zbig_hi);
+    } catch (const std::bad_alloc&) {
+        return;  // every segment is queried
     }
-    for (int t = 0; t < g.n_tris; ++t) {
-        const float4* v = &g.tris[3 * (size_t)t];
-        if (!is_big[t] && !(v[0].z == v[1].z && v[0].z == v[2].z)) continue;
-        is_big[t] = 1;
-        ++big.n_tris;
-        for (int c = 0; c < 3; ++c) big.tris.push_back(v[c]);
-    }
-    if (big.n_tris >= g.n_tris) return;  // no others: the z-gaps say all there is
     ++g_debug_counts.clearance_grids;
-    kp->n_zbig = occupied_z_slabs(big, kp->zbig_lo, kp->zbig_hi);
-    // padded boxes of the small triangles, and their bounds
-    auto box = [&](int t, float* lo, float* hi) {
-        const float4 a = g.tris[3 * (size_t)t], b = g.tris[3 * (size_t)t + 1], c = g.tris[3 * (size_t)t + 2];
-        const float v[3][3] = {{a.x, b.x, c.x}, {a.y, b.y, c.y}, {a.z, b.z, c.z}};
+    Box all = bounds[0];
+    for (const Box& b : bounds)
         for (int d = 0; d < 3; ++d) {
-            lo[d] = std::min(v[d][0], std::min(v[d][1], v[d][2]));
-            hi[d] = std::max(v[d][0], std::max(v[d][1], v[d][2]));
-            const float pad = 2e-5f * std::max(1.0f, std::max(std::fabs(lo[d]), std::fabs(hi[d])));
-            lo[d] -= pad;
-            hi[d] += pad;
+            all.lo[d] = std::min(all.lo[d], b.lo[d]);
+            all.hi[d] = std::max(all.hi[d], b.hi[d]);
         }
-    };
-    float blo[3] = {INFINITY, INFINITY, INFINITY}, bhi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int t = 0; t < g.n_tris; ++t) {
-        if (is_big[t]) continue;
-        float lo[3], hi[3];
-        box(t, lo, hi);
-        for (int d = 0; d < 3; ++d) {
-            blo[d] = std::min(blo[d], lo[d]);
-            bhi[d] = std::max(bhi[d], hi[d]);
-        }
-    }
     // cubic voxels where the bounds allow it, at least 8 along a thin axis (a height field's depth)
     double len[3], volume = 1.0;
     for (int d = 0; d < 3; ++d) {
-        len[d] = (double)bhi[d] - blo[d];
+        len[d] = (double)all.hi[d] - all.lo[d];
         if (!(len[d] > 0.0) || !std::isfinite(len[d])) return;
         volume *= len[d];
     }
@@ -504,9 +521,9 @@ void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std
         const int inner = (int)std::min((double)kClearanceAxis, std::max(8.0, std::ceil(len[d] / h)));
         const double w = len[d] / inner;
         n[d] = inner + 2 * kClearanceRim;
-        kp->small_lo[d] = blo[d];
-        kp->small_hi[d] = bhi[d];
-        kp->clear_o[d] = (float)(blo[d] - kClearanceRim * w);
+        kp->small_lo[d] = all.lo[d];
+        kp->small_hi[d] = all.hi[d];
+        kp->clear_o[d] = (float)(all.lo[d] - kClearanceRim * w);
         kp->clear_i[d] = (float)(1.0 / w);
     }
     const size_t nx = (size_t)n[0], ny = (size_t)n[1], nz = (size_t)n[2];
@@ -516,29 +533,35 @@ void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std
         return;  // every segment is queried
     }
     uint8_t* const D = clear->data();
-    for (int t = 0; t < g.n_tris; ++t) {
-        if (is_big[t]) continue;
-        float lo[3], hi[3];
-        int i0[3], i1[3];
-        box(t, lo, hi);
-        for (int d = 0; d < 3; ++d) {  // the kernel's arithmetic: voxel indices are monotone in the coordinate
-            const float a = (lo[d] - kp->clear_o[d]) * kp->clear_i[d], b = (hi[d] - kp->clear_o[d]) * kp->clear_i[d];
-            i0[d] = std::max(0, std::min(n[d] - 1, (int)std::floor(a)));
-            i1[d] = std::max(0, std::min(n[d] - 1, (int)std::floor(b)));
+    // The voxels of the boxes, each host thread a range of z. The kernel's arithmetic: voxel indices are monotone
+    // in the coordinate (cut off instead of rounded down, which differs below zero only, and there both are clamped).
+    parallel_parts(parts, [&](unsigned part) {
+        const int z0 = (int)(nz * part / parts), z1 = (int)(nz * (part + 1) / parts) - 1;
+        auto voxel = [&](int d, float x) {
+            return std::max(0, std::min(n[d] - 1, (int)((x - kp->clear_o[d]) * kp->clear_i[d])));
+        };
+        for (int t = 0; t < g.n_tris; ++t) {
+            if (is_big[t]) continue;
+            const Box& b = box[t];
+            const int k0 = std::max(z0, voxel(2, b.lo[2])), k1 = std::min(z1, voxel(2, b.hi[2]));
+            if (k0 > k1) continue;
+            const int i0 = voxel(0, b.lo[0]), i1 = voxel(0, b.hi[0]), j0 = voxel(1, b.lo[1]), j1 = voxel(1, b.hi[1]);
+            for (int k = k0; k <= k1; ++k)
+                for (int j = j0; j <= j1; ++j) {
+                    uint8_t* const row = D + ((size_t)k * ny + j) * nx;
+                    for (int i = i0; i <= i1; ++i) row[i] = 0;
+                }
         }
-        for (int k = i0[2]; k <= i1[2]; ++k)
-            for (int j = i0[1]; j <= i1[1]; ++j)
-                std::memset(D + ((size_t)k * ny + j) * nx + i0[0], 0, (size_t)(i1[0] - i0[0] + 1));
-    }
+    });
     // Chebyshev distance, one axis after the other: out[p] = min over q of max(|p - q|, in[q])
     const size_t step[3] = {1, nx, nx * ny};
+    const unsigned threads = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
     for (int d = 0; d < 3; ++d) {
         const size_t lines = nx * ny * nz / n[d], s = step[d];
         const int m = n[d];
-        const unsigned parts = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-        parallel_parts(parts, [&](unsigned part) {
+        parallel_parts(threads, [&](unsigned part) {
             uint8_t in[kClearanceAxis + 2 * kClearanceRim];
-            for (size_t l = lines * part / parts; l < lines * (part + 1) / parts; ++l) {
+            for (size_t l = lines * part / threads; l < lines * (part + 1) / threads; ++l) {
                 const size_t base = d == 0 ? l * nx : d == 1 ? (l / nx) * nx * ny + l % nx : l;
                 uint8_t* const line = D + base;
                 for (int p = 0; p < m; ++p) in[p] = line[(size_t)p * s];
@@ -556,7 +579,7 @@ void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std
     for (int d = 0; d < 3; ++d) kp->clear_n[d] = n[d];
 }
 
-void build_xy_grid(const GeomImage& g, GridImage* out, int tris_per_cell) {
+void build_xy_grid(const GeomImage& g, GridImage* out, int tris_per_cell, const std::function<void()>& big_known) {
     const double tpc = std::max(1, tris_per_cell);
     *out = GridImage();
     if (g.n_tris == 0) return;
@@ -692,6 +715,7 @@ void build_xy_grid(const GeomImage& g, GridImage* out, int tris_per_cell) {
             for (int c = 0; c < 3; ++c) out->big.push_back(g.tris[3 * (size_t)t + c]);
         }
     }
+    if (big_known) big_known();
     std::vector<unsigned int> count(nc, 0);
     for (int t = 0; t < g.n_tris; ++t) {
         if (is_big[t]) continue;

@@ -304,14 +304,28 @@ int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img
     kp.smem_next = smem_next;
     kp.n_nodes = geom.n_nodes;
     kp.n_tris = geom.n_tris;
-    // the occupied z-slabs and the xy grid read only the geometry: built side by side
+    // the occupied z-slabs and the xy grid read only the geometry, the clearance grid also the xy grid's list of big
+    // triangles: built side by side
     int n_zocc = 0;
     parallel_parts(2, [&](unsigned t) {
-        if (t == 1) n_zocc = occupied_z_slabs(geom, kp.zocc_lo, kp.zocc_hi);
-        else build_xy_grid(geom, &img->grid, opt.grid_cell_tris > 0 ? opt.grid_cell_tris : 12);
+        if (t == 1) {
+            n_zocc = occupied_z_slabs(geom, kp.zocc_lo, kp.zocc_hi);
+            return;
+        }
+        std::thread beside;
+        auto start_clearance = [&]() {
+            auto body = [&]() { build_clearance(geom, img->grid, &kp, &img->clear); };
+            try {
+                beside = std::thread(body);
+            } catch (...) {  // the system has no thread to give
+                body();
+            }
+        };
+        build_xy_grid(geom, &img->grid, opt.grid_cell_tris > 0 ? opt.grid_cell_tris : 12,
+                      clearance ? std::function<void()>(start_clearance) : nullptr);
+        if (beside.joinable()) beside.join();
     });
     kp.n_zocc = n_zocc;
-    if (clearance) build_clearance(geom, img->grid, &kp, &img->clear);
     kp.grid_x0 = img->grid.x0;
     kp.grid_y0 = img->grid.y0;
     kp.grid_icx = img->grid.icx;

@@ -3,6 +3,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <thread>
 #include <vector>
@@ -360,8 +361,9 @@ bool gpu_lbvh_topology(const std::vector<float>& cen, int n, int device, std::ve
 // bvh.cpp: merged z-intervals occupied by the triangles of `g` (at most kMaxZSlabs, conservative)
 int occupied_z_slabs(const GeomImage& g, float* lo, float* hi);
 
-// bvh.cpp: build the xy cell grid over the triangles of `g` (empty grid when there are none)
-void build_xy_grid(const GeomImage& g, GridImage* out, int tris_per_cell = 2);
+// bvh.cpp: build the xy cell grid over the triangles of `g` (empty grid when there are none); big_known is called
+// once the list of big triangles stands, with the cells still to be filled
+void build_xy_grid(const GeomImage& g, GridImage* out, int tris_per_cell = 2, const std::function<void()>& big_known = {});
 
 // bvh.cpp: clearance grid of the triangles of `g` that are neither big in `grid` nor horizontal; fills kp's clearance fields
 void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std::vector<uint8_t>* clear);
