@@ -58,18 +58,18 @@ __host__ __device__ __forceinline__ float tri_distance(float4 a, float4 b, float
                                                        float dx, float dy, float dz, unsigned& retests) {
     const float e1x = b.x - a.x, e1y = b.y - a.y, e1z = b.z - a.z;
     const float e2x = c.x - a.x, e2y = c.y - a.y, e2z = c.z - a.z;
-    const float px = dy * e2z - dz * e2y, py = dz * e2x - dx * e2z, pz = dx * e2y - dy * e2x;
-    const float det = e1x * px + e1y * py + e1z * pz;
+    const float px = diff2(dy, e2z, dz, e2y), py = diff2(dz, e2x, dx, e2z), pz = diff2(dx, e2y, dy, e2x);
+    const float det = dot3(e1x, e1y, e1z, px, py, pz);
     if (fabsf(det) < 1e-6f) return INFINITY;
     const float inv = 1.0f / det;
     const float sx = ox - a.x, sy = oy - a.y, sz = oz - a.z;
-    const float u = (sx * px + sy * py + sz * pz) * inv;
-    const float qx = sy * e1z - sz * e1y, qy = sz * e1x - sx * e1z, qz = sx * e1y - sy * e1x;
-    const float v = (dx * qx + dy * qy + dz * qz) * inv;
+    const float u = dot3(sx, sy, sz, px, py, pz) * inv;
+    const float qx = diff2(sy, e1z, sz, e1y), qy = diff2(sz, e1x, sx, e1z), qz = diff2(sx, e1y, sy, e1x);
+    const float v = dot3(dx, dy, dz, qx, qy, qz) * inv;
     const float w = 1.0f - u - v;
     const float band = c.w;  // per-triangle barycentric width of the FP64 re-test band
     if (u < -band || v < -band || w < -band) return INFINITY;
-    if (u > band && v > band && w > band) return (e2x * qx + e2y * qy + e2z * qz) * inv;
+    if (u > band && v > band && w > band) return dot3(e2x, e2y, e2z, qx, qy, qz) * inv;
     ++retests;
     return tri_distance_fp64(a, b, c, ox, oy, oz, dx, dy, dz);
 }

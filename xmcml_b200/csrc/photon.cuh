@@ -56,6 +56,23 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, const PhiloxKeys& k) {
 // 24-bit uniform in (0,1), exactly the value the FP64 oracle uses.
 __host__ __device__ __forceinline__ float u24(uint32_t x) { return fmaf((float)(x >> 8), 0x1p-24f, 0x1p-25f); }
 
+// Sums of products with the rounding of every term written out. Left to the compiler, which of two products is
+// rounded on its own differs from kernel to kernel with the registers at hand; a photon is walked by more than one
+// kernel, by which one is a matter of timing, and has to take the same path in each.
+__host__ __device__ __forceinline__ float mul_rn(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+// a b + c d, a b - c d, and the dot product of two vectors
+__host__ __device__ __forceinline__ float sum2(float a, float b, float c, float d) { return fmaf(a, b, mul_rn(c, d)); }
+__host__ __device__ __forceinline__ float diff2(float a, float b, float c, float d) { return fmaf(a, b, -mul_rn(c, d)); }
+__host__ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz) {
+    return fmaf(az, bz, sum2(ax, bx, ay, by));
+}
+
 #ifdef __CUDACC__
 // Reflectance of an interface for incidence cosine ci (0 < ci <= 1) from index ni into nt:
 // GetCriticalCos, ComputeTransmitCosine and ComputeFrenselReflectance of the reference
@@ -76,16 +93,15 @@ __device__ __forceinline__ float fresnel_reflectance(float ni, float nt, float c
         const double St = Ni * Si / Nt;
         if (St >= 1.0) return 1.0f;
         const double Ct = sqrt(1.0 - St * St);
-        const double cs = Ci * Ct - Si * St, cd = Ci * Ct + Si * St;
-        const double ss = Si * Ct + Ci * St, sd = Si * Ct - Ci * St;
-        return (float)(0.5 * sd * sd * (cd * cd + cs * cs) / (ss * ss * cd * cd));
+        const double pc = __dmul_rn(Si, St), ps = __dmul_rn(Ci, St);
+        const double cs = __fma_rn(Ci, Ct, -pc), cd = __fma_rn(Ci, Ct, pc);
+        const double ss = __fma_rn(Si, Ct, ps), sd = __fma_rn(Si, Ct, -ps);
+        return (float)(0.5 * sd * sd * __fma_rn(cd, cd, __dmul_rn(cs, cs)) / (ss * ss * cd * cd));
     }
     const float si = sqrtf(1.0f - ci * ci);
     const float st = ni * si / nt;
     if (st >= 1.0f) return 1.0f;
     const float ct = sqrtf(1.0f - st * st);
-    // Which product of each sum is rounded on its own is written out: left to the compiler it differs from
-    // kernel to kernel with the registers at hand, and a photon in ten million then takes the other branch.
     const float pc = __fmul_rn(si, st), ps = __fmul_rn(si, ct);
     const float cs = __fmaf_rn(ci, ct, -pc), cd = __fmaf_rn(ci, ct, pc);
     const float ss = __fmaf_rn(ci, st, ps), sd = __fmaf_rn(-ci, st, ps);

@@ -264,19 +264,19 @@ __device__ __forceinline__ void biased_spin(const KParams& P, const DevLayer& L,
     const float rx = ph.px - P.bias_ox, ry = ph.py - P.bias_oy, rz = ph.pz - P.bias_oz;
     const float ex = rx - P.bias_rx, ey = ry - P.bias_ry;
     const float az = rz - (P.bias_rz + ltr), bz = rz - (P.bias_rz - ltr - 2.0f * delta);
-    const float ia = rsqrtf(ex * ex + ey * ey + az * az), ib = rsqrtf(ex * ex + ey * ey + bz * bz);
+    const float ia = rsqrtf(dot3(ex, ey, az, ex, ey, az)), ib = rsqrtf(dot3(ex, ey, bz, ex, ey, bz));
     const float ca = ia * ia * ia, cb = ib * ib * ib;
-    float vx = ex * (cb - ca), vy = ey * (cb - ca), vz = bz * cb - az * ca;
-    const float vn = rsqrtf(vx * vx + vy * vy + vz * vz);
+    float vx = ex * (cb - ca), vy = ey * (cb - ca), vz = diff2(bz, cb, az, ca);
+    const float vn = rsqrtf(dot3(vx, vy, vz, vx, vy, vz));
     vx *= vn; vy *= vn; vz *= vn;
-    const float dot0 = ph.dx * vx + ph.dy * vy + ph.dz * vz;
+    const float dot0 = dot3(ph.dx, ph.dy, ph.dz, vx, vy, vz);
     float nx = ph.dx, ny = ph.dy, nz = ph.dz, p = 1.0f;
     for (uint32_t k = threadIdx.x & (kLanes - 1); k < kBiasMaxTrials; k += kLanes) {
         const uint4 r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter - 1u, 2u + k),
                                       P.keys);
         nx = ph.dx; ny = ph.dy; nz = ph.dz;
         hg_spin(L.hg_a, L.hg_b, L.hg_c, L.hg_d, L.hg_e, u24(r.x), u24(r.y), nx, ny, nz);
-        p = powf(fmaf(0.45f, 1.0f + (nx * vx + ny * vy + nz * vz), 0.1f), P.bias_eps);
+        p = powf(fmaf(0.45f, 1.0f + dot3(nx, ny, nz, vx, vy, vz), 0.1f), P.bias_eps);
         if constexpr (kLanes > 1) {
             const unsigned first = threadIdx.x & 31u & ~(kLanes - 1u);
             const unsigned group = (unsigned)((1ull << kLanes) - 1ull) << first;
@@ -360,33 +360,33 @@ __device__ __forceinline__ int cross_boundary(const KParams& P, const DevLayer* 
     // GetPlaneNormal (mcml_math.cpp:45-50), normalised
     const float e1x = a.x - b.x, e1y = a.y - b.y, e1z = a.z - b.z;
     const float e2x = a.x - c.x, e2y = a.y - c.y, e2z = a.z - c.z;
-    float nx = e1y * e2z - e1z * e2y, ny = e1z * e2x - e1x * e2z, nz = e1x * e2y - e1y * e2x;
-    const float nr = rsqrtf(nx * nx + ny * ny + nz * nz);
+    float nx = diff2(e1y, e2z, e1z, e2y), ny = diff2(e1z, e2x, e1x, e2z), nz = diff2(e1x, e2y, e1y, e2x);
+    const float nr = rsqrtf(dot3(nx, ny, nz, nx, ny, nz));
     nx *= nr; ny *= nr; nz *= nr;
     const int surf = __float_as_int(a.w);
     const int next = surf * MAX_LAYERS + ph.layer < P.smem_next ? (int)s_next[surf * MAX_LAYERS + ph.layer]
                                                                  : (int)__ldg(&P.next_layer[surf * MAX_LAYERS + ph.layer]);
     if (next < 0) return kCrossInvalid;
     const float ni = L.n, nt = s_layer[next].n;
-    const float dn = ph.dx * nx + ph.dy * ny + ph.dz * nz;
+    const float dn = dot3(ph.dx, ph.dy, ph.dz, nx, ny, nz);
     const float R = fresnel_reflectance(ni, nt, fabsf(dn));
     if (u_fresnel > R) {
         if (next == 0) return kCrossLeft;
         // RefractVector (mcml_kernel.cpp:595-616)
-        const float six = ni * ph.dx, siy = ni * ph.dy, siz = ni * ph.dz;
-        const float t1 = six * nx + siy * ny + siz * nz;
-        float t2 = sqrtf((nt * nt - ni * ni) / (t1 * t1) + 1.0f);
+        const float six = mul_rn(ni, ph.dx), siy = mul_rn(ni, ph.dy), siz = mul_rn(ni, ph.dz);
+        const float t1 = dot3(six, siy, siz, nx, ny, nz);
+        float t2 = sqrtf(diff2(nt, nt, ni, ni) / (t1 * t1) + 1.0f);
         t2 = (t2 - 1.0f) * t1;
-        float ox = six + t2 * nx, oy = siy + t2 * ny, oz = siz + t2 * nz;
-        const float on = rsqrtf(ox * ox + oy * oy + oz * oz);
+        float ox = fmaf(t2, nx, six), oy = fmaf(t2, ny, siy), oz = fmaf(t2, nz, siz);
+        const float on = rsqrtf(dot3(ox, oy, oz, ox, oy, oz));
         ph.dx = ox * on; ph.dy = oy * on; ph.dz = oz * on;
         ph.layer = next;
         ph.visited |= 1u << next;
     } else {
         // ReflectVector (mcml_kernel.cpp:582-593)
         const float t = 2.0f * dn;
-        float ox = ph.dx - t * nx, oy = ph.dy - t * ny, oz = ph.dz - t * nz;
-        const float on = rsqrtf(ox * ox + oy * oy + oz * oz);
+        float ox = fmaf(-t, nx, ph.dx), oy = fmaf(-t, ny, ph.dy), oz = fmaf(-t, nz, ph.dz);
+        const float on = rsqrtf(dot3(ox, oy, oz, ox, oy, oz));
         ph.dx = ox * on; ph.dy = oy * on; ph.dz = oz * on;
     }
     ph.excl = tri;
