@@ -465,12 +465,14 @@ int make_out_map(CUtensorMap* map, float* y, uint64_t rows, uint64_t n_out) {
     return XMC_OK;
 }
 
-template <int BN, class Epi>
-int set_smem_attr() {
-    static bool done = false;  // per template instance; set once per process (attribute is per function)
-    if (done) return XMC_OK;
-    XM_CUDA(cudaFuncSetAttribute(tc::gemm_kernel<BN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::smem_bytes(BN)));
-    done = true;
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device. `done`: one for each kernel.
+template <class F>
+int allow_smem(F kernel, int bytes, OncePerDevice& done) {
+    int device = 0;
+    XM_CUDA(cudaGetDevice(&device));
+    if (!done.pending(device)) return XMC_OK;
+    XM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done.set(device);
     return XMC_OK;
 }
 
@@ -480,7 +482,8 @@ int launch_gemm(const void* a, int rows_a, const void* b, int n, int k, int spli
                 cudaStream_t stream) {
     if (rows_a % tc::kBM || n % BN || k % (tc::kBK * splits) || splits < 1)
         return mfail(XMC_ERR_INVALID_INPUT, "gemm: shape not a multiple of the tile");
-    int st = set_smem_attr<BN, Epi>();
+    static OncePerDevice smem_set;
+    int st = allow_smem(tc::gemm_kernel<BN, Epi>, tc::smem_bytes(BN), smem_set);
     if (st) return st;
     CUtensorMap ma, mb;
     st = make_map(&ma, a, (uint64_t)rows_a, (uint64_t)k, tc::kBM);
@@ -596,17 +599,13 @@ bool fused_forward_ok(const xmc_mlp* m) {
 
 // Inference forward over `rows` rows of m->x into m->y with the fused kernel (mlp_fused.cuh).
 int enqueue_fused_forward(xmc_mlp* m, int rows) {
-    static bool attr = false;
-    if (!attr) {
-        XM_CUDA(cudaFuncSetAttribute(fused::mlp_forward_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     fused::kSmemBytes));
-        XM_CUDA(cudaFuncSetAttribute(fused::mlp_forward_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     fused::kSmemBytes));
-        attr = true;
-    }
+    static OncePerDevice smem_set[2];
+    int st = allow_smem(fused::mlp_forward_kernel<1>, fused::kSmemBytes, smem_set[0]);
+    if (!st) st = allow_smem(fused::mlp_forward_kernel<2>, fused::kSmemBytes, smem_set[1]);
+    if (st) return st;
     fused::Params p;
     std::memset(&p, 0, sizeof(p));
-    int st = make_map(&p.x, m->x, (uint64_t)rows, (uint64_t)kInPad, tc::kBM);
+    st = make_map(&p.x, m->x, (uint64_t)rows, (uint64_t)kInPad, tc::kBM);
     for (int l = 0; !st && l < m->L; ++l) {
         st = make_map(&p.w[l], m->w16[l], (uint64_t)m->out[l], (uint64_t)m->in[l], l < m->L - 1 ? m->spec.hidden : 256);
         p.bias[l] = m->b32[l];

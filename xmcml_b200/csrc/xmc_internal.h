@@ -393,6 +393,19 @@ struct DebugCounts {
 };
 extern DebugCounts g_debug_counts;  // capi.cpp
 
+// What has to be done once for each device of a process, such as raising a kernel's shared-memory limit (it belongs to
+// the function on one device). Two threads may both find it pending and do it.
+class OncePerDevice {
+  public:
+    bool pending(int device) const { return device >= 64 || !((done_.load(std::memory_order_acquire) >> device) & 1u); }
+    void set(int device) {
+        if (device < 64) done_.fetch_or(1ull << device, std::memory_order_release);
+    }
+
+  private:
+    std::atomic<unsigned long long> done_{0};  // devices from 64 on are never noted: it is done each time
+};
+
 // Keeps the caller's current CUDA device across an entry point: the device current on entry is
 // made current again when the guard goes out of scope (every return path), so an entry point that
 // selects a context's device does not move the caller's later work (or xmc_launch_omp, which runs
