@@ -683,25 +683,6 @@ int enqueue_forward(xmc_mlp* m, int rows, bool train, bool from_data_set = false
     return XMC_OK;
 }
 
-// What training alone needs, on the first call that trains: streams and events of the backward pass, the
-// minibatch's row numbers, and the split-K partials of every layer at the largest split any batch takes.
-int ensure_training(xmc_mlp* m) {
-    if (m->part[0]) return XMC_OK;
-    for (int k = 0; k < 2; ++k) {
-        if (!m->side[k]) XM_CUDA(cudaStreamCreateWithFlags(&m->side[k], cudaStreamNonBlocking));
-        if (!m->ev_side[k]) XM_CUDA(cudaEventCreateWithFlags(&m->ev_side[k], cudaEventDisableTiming));
-    }
-    size_t floats[kMaxLayers + 1] = {};
-    for (int l = 0; l < m->L; ++l) {
-        if (!m->ev_dz[l]) XM_CUDA(cudaEventCreateWithFlags(&m->ev_dz[l], cudaEventDisableTiming));
-        floats[l + 1] = floats[l] + (size_t)m->out[l] * m->in[l] * std::max(1, 128 / (m->out[l] / tc::kBM));
-    }
-    if (!m->src) XM_CUDA(cudaMalloc(&m->src, sizeof(int) * (size_t)m->cap));
-    XM_CUDA(cudaMalloc(&m->part[0], sizeof(float) * floats[m->L]));
-    for (int l = 1; l < m->L; ++l) m->part[l] = m->part[0] + floats[l];
-    return XMC_OK;
-}
-
 // Backward pass after enqueue_forward(train): per-layer partial weight gradients into m->part, bias gradients
 // into m->gb. The data gradients are one chain; each layer's weight and bias gradients hang off it and run on
 // a stream of their own.
@@ -830,7 +811,22 @@ extern "C" int xmc_mlp_create(const xmc_mlp_spec* spec, xmc_mlp** out) {
     XM_TRY(cudaMalloc(&m->d_loss, sizeof(float) * (m->loss_cap + 1)));
     XM_TRY(cudaMemset(m->d_err, 0, sizeof(int)));
     XM_TRY(cudaMemset(m->d_step, 0, 2 * sizeof(int)));
+    // Training's buffers too, so that no training call of a model that was made fails for want of memory: streams and
+    // events of the backward pass, the minibatch's row numbers, and the split-K partials of every layer at the
+    // largest split any batch takes.
+    for (int k = 0; k < 2; ++k) {
+        XM_TRY(cudaStreamCreateWithFlags(&m->side[k], cudaStreamNonBlocking));
+        XM_TRY(cudaEventCreateWithFlags(&m->ev_side[k], cudaEventDisableTiming));
+    }
+    size_t part_at[kMaxLayers + 1] = {};
+    for (int l = 0; l < m->L; ++l) {
+        XM_TRY(cudaEventCreateWithFlags(&m->ev_dz[l], cudaEventDisableTiming));
+        part_at[l + 1] = part_at[l] + (size_t)m->out[l] * m->in[l] * std::max(1, 128 / (m->out[l] / tc::kBM));
+    }
+    XM_TRY(cudaMalloc(&m->part[0], sizeof(float) * part_at[m->L]));
+    for (int l = 1; l < m->L; ++l) m->part[l] = m->part[0] + part_at[l];
     const size_t R = (size_t)m->cap;
+    XM_TRY(cudaMalloc(&m->src, sizeof(int) * R));
     for (int l = 0; l < m->L; ++l) {
         const size_t n = (size_t)m->out[l] * m->in[l];
         XM_TRY(cudaMalloc(&m->w32[l], sizeof(float) * n));
@@ -1061,8 +1057,7 @@ extern "C" int xmc_mlp_gradients(xmc_mlp* m, const float* x, const float* t, int
     int st = check_rows(m, rows);
     if (st) return st;
     XM_CUDA(cudaSetDevice(m->spec.device));
-    st = ensure_training(m);
-    if (!st) st = upload_inputs(m, x, rows, rows, true);
+    st = upload_inputs(m, x, rows, rows, true);
     if (st) return st;
     XM_CUDA(cudaMemcpyAsync(m->t, t, sizeof(float) * (size_t)rows * m->spec.n_out, cudaMemcpyHostToDevice, m->stream));
     // loss slot: loss[step + ... ] uses *d_step; use slot (current step) after zeroing it
@@ -1123,8 +1118,6 @@ extern "C" int xmc_mlp_train(xmc_mlp* m, int steps, int batch, float lr, float b
     int st = check_rows(m, batch);
     if (st) return st;
     XM_CUDA(cudaSetDevice(m->spec.device));
-    st = ensure_training(m);
-    if (st) return st;
     int step0 = 0;
     XM_CUDA(cudaMemcpy(&step0, m->d_step, sizeof(int), cudaMemcpyDeviceToHost));
     if (step0 + steps >= m->loss_cap) return mfail(XMC_ERR_RANGE, "too many training steps for the loss log");
