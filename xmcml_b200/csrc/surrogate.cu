@@ -511,6 +511,7 @@ struct xmc_mlp {
     int in[kMaxLayers], out[kMaxLayers];   // padded dimensions
     int valid_out[kMaxLayers];             // rows of W that are real (n_out for the last layer)
     int cap = 0;                    // row capacity
+    int sms = 0;                    // of its device
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     int* d_err = nullptr;
@@ -577,10 +578,10 @@ void free_mlp(xmc_mlp* m) {
     delete m;
 }
 
-// Widest tile that still gives the chip's SMs a CTA each, else the narrowest: the tile width changes no sum.
-int tile_width(int rows_a, int n, int splits) {
+// Widest tile that still gives the device's `sms` SMs a CTA each, else the narrowest: the tile width changes no sum.
+int tile_width(int rows_a, int n, int splits, int sms) {
     for (int bn = 256; bn > 64; bn /= 2)
-        if (n % bn == 0 && (rows_a / tc::kBM) * (n / bn) * splits >= 148) return bn;
+        if (n % bn == 0 && (rows_a / tc::kBM) * (n / bn) * splits >= sms) return bn;
     return 64;
 }
 
@@ -618,8 +619,7 @@ int enqueue_fused_forward(xmc_mlp* m, int rows) {
     p.n_tiles = rows / tc::kBM;
     p.n_out = m->spec.n_out;
     p.err = m->d_err;
-    int sms = 0;
-    XM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->spec.device));
+    const int sms = m->sms;
     // no more tiles than SMs: one tile per CTA; where the SMs also suffice for every output chunk of every tile, a
     // CTA takes one of those
     p.split = p.n_tiles * p.out_chunks <= sms;
@@ -633,12 +633,12 @@ int enqueue_fused_forward(xmc_mlp* m, int rows) {
 
 // D = A . B^T with the widest tile that fills the chip.
 template <class Epi>
-int launch_gemm_wide(const void* a, int rows_a, const void* b, int n, int k, int splits, const Epi& epi, int* err,
+int launch_gemm_wide(const xmc_mlp* m, const void* a, int rows_a, const void* b, int n, int k, int splits, const Epi& epi,
                      cudaStream_t stream) {
-    switch (tile_width(rows_a, n, splits)) {
-        case 256: return launch_gemm<256>(a, rows_a, b, n, k, splits, epi, err, stream);
-        case 128: return launch_gemm<128>(a, rows_a, b, n, k, splits, epi, err, stream);
-        default: return launch_gemm<64>(a, rows_a, b, n, k, splits, epi, err, stream);
+    switch (tile_width(rows_a, n, splits, m->sms)) {
+        case 256: return launch_gemm<256>(a, rows_a, b, n, k, splits, epi, m->d_err, stream);
+        case 128: return launch_gemm<128>(a, rows_a, b, n, k, splits, epi, m->d_err, stream);
+        default: return launch_gemm<64>(a, rows_a, b, n, k, splits, epi, m->d_err, stream);
     }
 }
 
@@ -653,7 +653,7 @@ int enqueue_forward(xmc_mlp* m, int rows, bool train, bool from_data_set = false
         int s;
         if (l < m->L - 1) {
             EpiHidden e{m->b32[l], m->a[l], m->out[l], train ? m->z[l] : nullptr, train ? m->at[l] : nullptr, rows};
-            s = launch_gemm_wide(a_in, rows, m->w16[l], m->out[l], k, 1, e, m->d_err, st);
+            s = launch_gemm_wide(m, a_in, rows, m->w16[l], m->out[l], k, 1, e, st);
         } else {
             EpiOut e{};
             e.bias = m->b32[l];
@@ -676,7 +676,7 @@ int enqueue_forward(xmc_mlp* m, int rows, bool train, bool from_data_set = false
                 e.y = m->y;
                 e.ldy = m->spec.n_out;
             }
-            s = launch_gemm_wide(a_in, rows, m->w16[l], m->out[l], k, 1, e, m->d_err, st);
+            s = launch_gemm_wide(m, a_in, rows, m->w16[l], m->out[l], k, 1, e, st);
         }
         if (s) return s;
     }
@@ -692,7 +692,7 @@ int enqueue_backward(xmc_mlp* m, int rows) {
         XM_CUDA(cudaEventRecord(m->ev_dz[l], st));  // dZ_l is ready
         if (l > 0) {
             EpiBwd e{m->z[l - 1], m->out[l - 1], m->dz[l - 1], m->dzt[l - 1], rows};
-            const int s = launch_gemm_wide(m->dz[l], rows, m->w16t[l], m->in[l], m->out[l], 1, e, m->d_err, st);
+            const int s = launch_gemm_wide(m, m->dz[l], rows, m->w16t[l], m->in[l], m->out[l], 1, e, st);
             if (s) return s;
         }
         // bias gradient, then the weight gradient dW = dZ^T . A_{l-1}, split over rows. The first layer's, the last
@@ -702,7 +702,7 @@ int enqueue_backward(xmc_mlp* m, int rows) {
         XM_CUDA(cudaGetLastError());
         const bf16* bt = l == 0 ? m->xt : m->at[l - 1];
         EpiF32 e{m->part[l], m->in[l], (size_t)m->out[l] * m->in[l]};
-        const int s = launch_gemm_wide(m->dzt[l], m->out[l], bt, m->in[l], rows, wgrad_splits(m, l, rows), e, m->d_err, m->side[l & 1]);
+        const int s = launch_gemm_wide(m, m->dzt[l], m->out[l], bt, m->in[l], rows, wgrad_splits(m, l, rows), e, m->side[l & 1]);
         if (s) return s;
     }
     for (int k = 0; k < std::min(2, m->L); ++k) {
@@ -802,6 +802,7 @@ extern "C" int xmc_mlp_create(const xmc_mlp_spec* spec, xmc_mlp** out) {
         }                                                                                        \
     } while (0)
     XM_TRY(cudaSetDevice(s.device));
+    XM_TRY(cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, s.device));
     XM_TRY(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
     XM_TRY(cudaEventCreate(&m->ev[0]));
     XM_TRY(cudaEventCreate(&m->ev[1]));
@@ -892,7 +893,7 @@ extern "C" int xmc_mlp_set_params(xmc_mlp* m, const float* p) {
         XM_CUDA(cudaMemset(m->vw[l], 0, sizeof(float) * w.size()));
         XM_CUDA(cudaMemset(m->mb[l], 0, sizeof(float) * b.size()));
         XM_CUDA(cudaMemset(m->vb[l], 0, sizeof(float) * b.size()));
-        refresh_kernel<<<148, 256, 0, m->stream>>>(m->w32[l], m->out[l], m->in[l], m->w16[l], m->w16t[l]);
+        refresh_kernel<<<m->sms, 256, 0, m->stream>>>(m->w32[l], m->out[l], m->in[l], m->w16[l], m->w16t[l]);
         XM_CUDA(cudaGetLastError());
         in = vo;
     }
