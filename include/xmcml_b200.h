@@ -237,10 +237,11 @@ typedef struct xmc_options {
     int32_t  trajectory_log;       /* XMC_DETECTOR_TRAJ: z-plane crossings logged per resident thread
                                     * (0 = 4096, at most 65536; -1 = no log, every detected photon
                                     * is replayed)                                                 */
-    int32_t  query_batch;          /* lanes of a warp that wait for a ray query, glass, or the end of
-                                    * their photon while the others go on, before the warp takes those
-                                    * steps together (0 = 12), in either query scheme. A scheduling
-                                    * choice: tallies are the same bit for bit                     */
+    int32_t  query_batch;          /* cooperative ray queries: lanes of a warp that wait for a query,
+                                    * glass, or the end of their photon while the others go on, before
+                                    * the warp takes those steps together (0 = 12; fewer count as 12;
+                                    * lane by lane always 12). A scheduling choice: tallies are the
+                                    * same bit for bit                                             */
     int32_t  grid_cell_tris;       /* triangles per cell the xy grid of short ray queries aims at (0 = 12;
                                     * larger: coarser cells, fewer queries fall back to the BVH). A
                                     * speed choice: tallies are the same bit for bit              */
@@ -330,11 +331,11 @@ int xmc_destroy(xmc_context* ctx);
  * Builds the device image of `input` under `base` (its flags, device and semantics are kept) and
  * times `sample_photons` photons (0 = 1e6) under every candidate: xy-grid density grid_cell_tris
  * {2, 8, 16, 32} triangles per cell, block size {256, 512} at the occupancy maximum, photon ids a warp
- * claims from the dispenser at a time {32, 64}, query_batch {8, 12, 16}, and the ray-query scheme
- * (warp-cooperative, or lane by lane with XMC_LANE_QUERIES): 96 candidates, each timed once, the four
- * fastest twice more on other photons. *best gets `base` with the fastest one, *best_ms (may be NULL) its
- * best kernel time. Every candidate gives bit-identical tallies: a photon's random numbers, its candidate triangles' arithmetic and the choice among equal
- * distances (the lower triangle index) do not depend on them. */
+ * claims from the dispenser at a time {32, 64}, and the ray-query scheme (warp-cooperative with query_batch
+ * {12, 16}, or lane by lane with XMC_LANE_QUERIES): 48 candidates, each timed once, the four fastest twice more
+ * on other photons. *best gets `base` with the fastest one, *best_ms (may be NULL) its best kernel time. Every
+ * candidate gives bit-identical tallies: a photon's random numbers, its candidate triangles' arithmetic and the
+ * choice among equal distances (the lower triangle index) do not depend on them. */
 int xmc_autotune(const InputInfo* input, const xmc_options* base, uint64_t sample_photons, xmc_options* best,
                  double* best_ms);
 
@@ -455,6 +456,9 @@ void xmc_debug_free_depths(float z_top, float z_bot, float inv_mut, float* zlo, 
 /* Counts since the library was loaded, into out[0..max_count); returns how many there are. [0] transport and
  * batch runs that a tail kernel walked whole; [1] clearance grids built. Used by the test suites. */
 int xmc_debug_counts(uint64_t* out, int max_count);
+
+/* The lanes that wait for a general step under `opt` (query_batch above). Used by the test suites. */
+int xmc_debug_waiting_lanes(const xmc_options* opt);
 
 /* The launch shapes that xmc_autotune times on each grid density, made from `base`, into out[0..max_count);
  * returns how many there are. Used by the test suites. */

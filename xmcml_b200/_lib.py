@@ -64,6 +64,7 @@ def load(path: str | None = None) -> C.CDLL:
                                         P(C.c_float), P(C.c_int), P(C.c_float), C.c_int]),
         "xmc_debug_free_depths": (None, [C.c_float, C.c_float, C.c_float, P(C.c_float), P(C.c_float)]),
         "xmc_debug_counts": (C.c_int, [P(C.c_uint64), C.c_int]),
+        "xmc_debug_waiting_lanes": (C.c_int, [P(S.XmcOptions)]),
         "xmc_debug_launch_shapes": (C.c_int, [P(S.XmcOptions), P(S.XmcOptions), C.c_int]),
         "xmc_run_noalloc": (C.c_int, [P(S.InputInfo), P(S.XmcOptions), C.c_uint64, C.c_uint64, C.c_uint64,
                                       C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
@@ -118,7 +119,7 @@ EXPORTS = [
     "xmc_cancel", "xmc_read_maps", "xmc_destroy", "xmc_launch", "xmc_launch_omp", "xmc_init_output", "xmc_free_output",
     "xmc_parse_input_file", "xmc_parse_surface_file", "xmc_free_input", "xmc_write_output_file",
     "xmc_specular_reflectance", "xmc_philox4x32_10", "xmc_layout_offsets", "xmc_device_philox",
-    "xmc_generate_bvh_tree", "xmc_free_bvh_tree", "xmc_debug_nearest", "xmc_debug_free_depths", "xmc_debug_counts", "xmc_debug_launch_shapes",
+    "xmc_generate_bvh_tree", "xmc_free_bvh_tree", "xmc_debug_nearest", "xmc_debug_free_depths", "xmc_debug_counts", "xmc_debug_waiting_lanes", "xmc_debug_launch_shapes",
     "xmc_run_noalloc",
     "xmc_batch_validate", "xmc_batch_create", "xmc_batch_run", "xmc_batch_read_tallies", "xmc_batch_set_tuning",
     "xmc_batch_get_tuning", "xmc_batch_autotune", "xmc_batch_destroy",

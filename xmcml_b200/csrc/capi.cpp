@@ -147,6 +147,16 @@ static int validate(const InputInfo* in, const xmc_options& opt) {
     return XMC_OK;
 }
 
+// Lanes of a warp that wait for a general step before it is taken. Cooperative queries: query_batch, but never fewer
+// than 12, which is faster than any smaller number on every scene (5e5 photons, ms at 1 / 4 / 8 / 12 lanes: planar
+// stack 24 / 19 / 17 / 17, glass cover 13 / 10 / 8.1 / 7.3, height field 37 / 28 / 24 / 23, ellipsoid 39 / 33 / 29 / 28,
+// biased 16 / 13 / 11.7 / 10.9); more are the caller's choice (glass cover, 16: 7.0). Lane by lane there are no rounds
+// of queries to collect: always 12 (16: within 5 % either way, 32: 17 -> 125 ms on the planar stack).
+static int waiting_lanes(const xmc_options& opt) {
+    if ((opt.flags & XMC_LANE_QUERIES) || opt.query_batch <= 12) return 12;
+    return std::min(32, (int)opt.query_batch);
+}
+
 int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img, bool clearance) {
     xmc_options opt;
     xmc_default_options(&opt);
@@ -334,7 +344,7 @@ int prepare_image(const InputInfo* in, const xmc_options* opt_in, HostImage* img
     kp.grid_ny = img->grid.ny;
     kp.n_big = (int)(img->grid.big.size() / 4);
     kp.coop_query = (opt.flags & XMC_LANE_QUERIES) ? 0 : 1;
-    kp.query_batch = opt.query_batch > 0 ? std::min(32, (int)opt.query_batch) : 12;
+    kp.query_batch = waiting_lanes(opt);
     const int block = opt.block_size > 0 ? opt.block_size : 512;
     img->smem_bytes = smem_layout(nd, smem_nodes, smem_tris, smem_next, kp.coop_query ? block / 32 : 0);
     // ---- biasing (mcml_kernel.cpp:325-440) ----
@@ -998,15 +1008,13 @@ static const int kTuneDensities[] = {2, 8, 16, 32};
 static std::vector<xmc_options> launch_shapes(const xmc_options& base) {
     const int blocks[] = {256, 512};
     const int chunks[] = {32, 64};
-    // lanes that wait for a general step, in either query scheme. Not 1 (1e6 photons, ms at 1 / 8 / 12 / 16 lanes:
-    // height field 70 / 41 / 39 / 41, lane by lane 105 / 66 / 62 / 61; ellipsoid 71 / 50 / 48 / 50, 94 / 71 / 68 / 70;
-    // glass cover 30 / 18 / 16 / 15, 34 / 21 / 18 / 16)
-    const int batches[] = {8, 12, 16};
+    const int batches[] = {12, 16};  // cooperative (waiting_lanes)
     std::vector<xmc_options> shapes;
     for (int coop = 1; coop >= 0; --coop)
         for (int b : blocks)
             for (int ch : chunks)
                 for (int qb : batches) {
+                    if (!coop && qb != batches[0]) continue;
                     xmc_options c = base;
                     c.block_size = b;
                     c.blocks_per_sm = 0;
@@ -1017,6 +1025,8 @@ static std::vector<xmc_options> launch_shapes(const xmc_options& base) {
                 }
     return shapes;
 }
+
+int xmc_debug_waiting_lanes(const xmc_options* opt) { return waiting_lanes(*opt); }
 
 int xmc_debug_launch_shapes(const xmc_options* base, xmc_options* out, int max_count) {
     const std::vector<xmc_options> shapes = launch_shapes(*base);
@@ -1059,7 +1069,7 @@ int xmc_autotune(const InputInfo* input, const xmc_options* base, uint64_t sampl
         img.kp.flags = c.flags;
         img.kp.chunk = c.photons_per_chunk;
         img.kp.coop_query = (c.flags & XMC_LANE_QUERIES) ? 0 : 1;
-        img.kp.query_batch = c.query_batch;
+        img.kp.query_batch = waiting_lanes(c);
         img.smem_bytes = smem_layout(img.n_dets, img.kp.smem_nodes, img.kp.smem_tris, img.kp.smem_next,
                                      img.kp.coop_query ? c.block_size / 32 : 0);
         return img;

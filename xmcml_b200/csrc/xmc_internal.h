@@ -180,7 +180,7 @@ struct KParams {
     int coop_query;           // 1: grid queries run warp-cooperatively (WarpQuery scratch per warp in
                               // shared memory); 0: each lane walks its own cells
     int query_batch;          // a warp takes its lanes' general steps together once this many lanes wait for one
-                              // (or every live lane does), in either query scheme
+                              // (or every live lane does), in either query scheme; at least 12 (capi.cpp waiting_lanes)
     // clearance grid (clear_n[0] == 0: none)
     const uint8_t* clear;
     float clear_o[3], clear_i[3];     // origin, 1 / voxel size
