@@ -359,7 +359,9 @@ int xmc_launch(const InputInfo* input, OutputInfo* output, uint64_t seed,
  * The device copy of the model (BVH nodes, triangles, layer transitions, detectors, xy cell grid)
  * and the photon-id dispenser live in one static device array of XMC_NOALLOC_SCRATCH_BYTES (8 MiB)
  * that every GPU loading the library holds until exit; a model that needs more is rejected with
- * XMC_ERR_RANGE (a mesh of up to roughly 50,000 triangles fits). The first call on a device is its
+ * XMC_ERR_RANGE (a mesh of up to roughly 50,000 triangles fits). What is left of the array holds the tables
+ * that speed alone depends on (cooperative queries, the tail kernel's list, the clearance grid), as far as they
+ * fit. The first call on a device is its
  * set-up: it looks up that array's device address (cudaGetSymbolAddress) and keeps it, so make that
  * first call before any stream capture starts on the device. All calls share the array and it keeps
  * the last call's contents: calls that overlap on the GPU (on different streams or threads) race and

@@ -1,5 +1,6 @@
-"""xmc_run_noalloc stages no clearance grid, so it builds none: the call of a model that exceeds its scratch, which
-ends after the host image is built and before the GPU is touched, leaves the count of built grids as it is."""
+"""xmc_run_noalloc builds a clearance grid only for runs that pay for it: the call of a model that exceeds its scratch,
+which ends after the host image is built and before the GPU is touched, leaves the count of built grids as it is
+with few photons and raises it with many."""
 import ctypes as C
 
 import numpy as np
@@ -14,15 +15,16 @@ def _grids_built(lib):
     return v[1]
 
 
-def test_noalloc_builds_no_clearance_grid(tmp_path):
+def test_short_runs_build_no_clearance_grid(tmp_path):
     lib = _lib.load()
     m = api.Model(*scenes.height_field_tissue(photons=1).write(str(tmp_path), "big"))
     before = _grids_built(lib)
     opts, dummy = api.options(), C.c_void_p(1)
-    assert lib.xmc_run_noalloc(C.byref(m.info), C.byref(opts), 1, 0, 10, dummy, dummy, dummy, dummy, None) == S.XMC_ERR_RANGE
-    assert _grids_built(lib) == before
+    for n, grids in ((10, 0), (39_999, 0), (40_000, 1)):
+        assert lib.xmc_run_noalloc(C.byref(m.info), C.byref(opts), 1, 0, n, dummy, dummy, dummy, dummy, None) == S.XMC_ERR_RANGE
+        assert _grids_built(lib) == before + grids
     f, i = np.zeros(1, np.float32), np.zeros(1, np.int32)
     pf, pi = C.POINTER(C.c_float), C.POINTER(C.c_int)
     _lib.check(lib.xmc_debug_nearest(C.byref(m.info), 0, f.ctypes.data_as(pf), 0.0, 1.0, f.ctypes.data_as(pf),
                                      i.ctypes.data_as(pi), None, 4))
-    assert _grids_built(lib) == before + 1
+    assert _grids_built(lib) == before + 2

@@ -20,6 +20,10 @@ namespace {
 
 constexpr size_t kNoAllocScratchBytes = XMC_NOALLOC_SCRATCH_BYTES;
 constexpr size_t kAlign = 256;
+// Photons of a run from which on its clearance grid is built and staged, which each call pays for again (1.3 ms on an
+// ellipsoid of 5,120 triangles, 2.5 ms on a height field of 2 x 64 x 64 cells): with it 4e4 photons take 15.5 ms
+// there instead of 16.7, 3e4 17 instead of 14.
+constexpr uint64_t kClearanceRun = 40000;
 
 // The scratch array. In host code `g_noalloc_scratch` is only a host-side stand-in for the symbol;
 // its device address comes from cudaGetSymbolAddress (noalloc_scratch_address below).
@@ -70,10 +74,8 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     xmc_default_options(&o);
     if (opt && opt->struct_size) std::memcpy(&o, opt, std::min((size_t)opt->struct_size, sizeof(o)));
     o.flags &= ~XMC_GPU_BVH;
-    o.flags |= XMC_LANE_QUERIES;  // the cooperative query's entry records would need more scratch
-    // no clearance grid: it is not staged, and each call would build it again (height field of 2 x 64 x 64 cells:
-    // 13.6 -> 11.1 ms per call of 10 photons)
-    int st = prepare_image(input, &o, &img, false);
+    if (o.block_size <= 0) o.block_size = 256;
+    int st = prepare_image(input, &o, &img, n_photons >= kClearanceRun);
     if (st) return st;
     if (img.kp.use_bias) {
         set_error("xmc_run_noalloc: biasing needs weight tables this entry point does not stage");
@@ -85,8 +87,9 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     }
     const GeomImage& geom = img.geom;
 
-    // scratch layout: [dispenser u64 | status int | cancel int] [nodes] [triangles] [transition table]
-    // [detectors] [grid cells] [cell z-intervals] [grid entries] [big triangles]
+    // scratch layout: [dispenser u64 | status int | .. | at 64: tail counts] [nodes] [triangles] [transition table]
+    // [detectors] [grid cells] [cell z-intervals] [grid entries] [big triangles], and what speed alone depends on,
+    // each where there is room left for it: [entries per z-interval] [tail list] [clearance grid]
     const size_t b_nodes = sizeof(float4) * geom.nodes.size();
     const size_t b_tris = sizeof(float4) * geom.tris.size();
     const size_t b_next = img.next.size();
@@ -157,7 +160,7 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
 
     int sms = 0, occ = 0;
     NA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    c.block = img.opt.block_size > 0 ? img.opt.block_size : 256;
+    c.block = img.opt.block_size;
     if (c.block % 32 != 0 || c.block > 1024) {
         set_error("xmc_run_noalloc: block_size must be a multiple of 32 <= 1024");
         return XMC_ERR_INVALID_INPUT;
@@ -170,6 +173,35 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     c.blocks_per_sm = img.opt.blocks_per_sm > 0 ? std::min(img.opt.blocks_per_sm, occ) : occ;
     c.grid = sms * c.blocks_per_sm;
 
+    size_t used = need;
+    auto room = [&](size_t bytes, size_t* at) {
+        if (used + align_up(bytes) > kNoAllocScratchBytes) return false;
+        *at = used;
+        used += align_up(bytes);
+        return true;
+    };
+    // cooperative queries; lane by lane without their table
+    const size_t b_runs = sizeof(uint32_t) * img.grid.cell_runs.size();
+    size_t o_runs = 0, o_tail = 0, o_clear = 0;
+    if (kp.coop_query && room(b_runs, &o_runs)) kp.cell_runs = reinterpret_cast<const uint32_t*>(scratch + o_runs);
+    else kp.coop_query = 0;
+    // The tail kernel, with a list for what the transport kernel's warps hand over, or for runs of up to half as many
+    // photons as the grid has threads, which it walks whole. 4e4 / 6e4 photons lost at the Area's faces, whole and
+    // through both kernels: ellipsoid of 1,280 triangles 13.5 / 16.5 and 12.9 / 13.4 ms, planar stack 2.9 / 3.7 and
+    // 2.4 / 2.5; 3e4 photons, ellipsoid of 5,120: 14.4 and 17.2.
+    int tail_occ = 0, tail_photons = 0;
+    NA_CK(tail_occupancy(kp, &c.tail_smem, &tail_occ, &tail_photons));
+    c.tail_takes_small_runs = n_photons <= (unsigned long long)c.grid * c.block / 2;
+    const size_t b_tail = c.tail_takes_small_runs ? 0 : sizeof(TailPhoton) * (size_t)c.grid * (c.block / 32) * kTailLanes;
+    if (tail_occ > 0 && room(b_tail, &o_tail)) {
+        c.tail_grid = sms * tail_occ;
+        kp.tail_count = reinterpret_cast<unsigned*>(scratch + 64);
+        kp.tail_next = kp.tail_count + 1;
+        kp.tail = reinterpret_cast<TailPhoton*>(scratch + o_tail);
+    }
+    if (kp.clear_n[0] && room(img.clear.size(), &o_clear)) kp.clear = scratch + o_clear;
+    else kp.clear_n[0] = 0;  // every segment outside the z-gaps is queried
+
     // the scratch keeps the previous call's contents: the dispenser and status start at zero
     NA_CK(cudaMemsetAsync(scratch, 0, kAlign, c.stream));
     if (b_nodes) NA_CK(cudaMemcpyAsync(scratch + o_nodes, geom.nodes.data(), b_nodes, cudaMemcpyHostToDevice, c.stream));
@@ -180,6 +212,10 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     if (b_cell_z) NA_CK(cudaMemcpyAsync(scratch + o_cell_z, img.grid.cell_z.data(), b_cell_z, cudaMemcpyHostToDevice, c.stream));
     if (b_entries)
         NA_CK(cudaMemcpyAsync(scratch + o_entries, img.grid.entries.data(), b_entries, cudaMemcpyHostToDevice, c.stream));
+    if (kp.coop_query && b_runs)
+        NA_CK(cudaMemcpyAsync(scratch + o_runs, img.grid.cell_runs.data(), b_runs, cudaMemcpyHostToDevice, c.stream));
+    if (kp.clear_n[0])
+        NA_CK(cudaMemcpyAsync(scratch + o_clear, img.clear.data(), img.clear.size(), cudaMemcpyHostToDevice, c.stream));
     if (b_big) NA_CK(cudaMemcpyAsync(scratch + o_big, img.grid.big.data(), b_big, cudaMemcpyHostToDevice, c.stream));
     const size_t nd = (size_t)std::max(1, img.n_dets);
     NA_CK(cudaMemsetAsync(d_absorption, 0, sizeof(unsigned long long) * (size_t)img.grid_size, c.stream));
