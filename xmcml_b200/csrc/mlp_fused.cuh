@@ -105,7 +105,17 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 
 // layer geometry: MMA N of one chunk, chunks, 64-column k-blocks
 __device__ __forceinline__ int layer_n(const Params& p, int l) { return l < p.L - 1 ? p.hidden : 256; }
-__device__ __forceinline__ int layer_chunks(const Params& p, int l) { return l < p.L - 1 || p.split ? 1 : p.out_chunks; }
+// p.split, which only one slot can have: the kernel of two slots carries no test of it (19,072 and 65,536 rows,
+// 15-256-4096: 125.5 and 281.9 us with, 124.8 and 278.7 us without)
+template <int kSlots>
+__device__ __forceinline__ bool is_split(const Params& p) {
+    if constexpr (kSlots == 1) return p.split != 0;
+    else return false;
+}
+template <int kSlots>
+__device__ __forceinline__ int layer_chunks(const Params& p, int l) {
+    return l < p.L - 1 || is_split<kSlots>(p) ? 1 : p.out_chunks;
+}
 __device__ __forceinline__ int layer_kblocks(const Params& p, int l) { return l == 0 ? 1 : p.hidden / 64; }
 
 // Epilogue of 32 accumulator columns of a hidden layer: bias + SiLU, written as BF16 (4 chunks of 16 B)
@@ -182,6 +192,7 @@ struct SlotCount {
 // chunk) of one tile; a tile has L - 1 + out_chunks jobs. Slot s takes this CTA's tiles s, s + 2,
 // s + 4, ... (tile blockIdx.x + i gridDim.x for the CTA's i-th tile); the slots alternate job by job
 // while both have tiles left, and each moves on to its next tile on its own.
+template <int kSlots>
 struct JobOrder {
     int i0, l0, c0, i1, l1, c1;  // per slot: the CTA's tile ordinal, layer and chunk of its next job
     int my_tiles, turn;
@@ -193,10 +204,10 @@ struct JobOrder {
         s = a0 && a1 ? turn : (a0 ? 0 : 1);
         turn = s ^ 1;
         int i = s ? i1 : i0, l = s ? l1 : l0, c = s ? c1 : c0;
-        tile = p.split ? (int)blockIdx.x / p.out_chunks : (int)blockIdx.x + i * (int)gridDim.x;
+        tile = is_split<kSlots>(p) ? (int)blockIdx.x / p.out_chunks : (int)blockIdx.x + i * (int)gridDim.x;
         layer = l;
-        chunk = p.split && l == p.L - 1 ? (int)blockIdx.x % p.out_chunks : c;
-        if (++c == layer_chunks(p, l)) {
+        chunk = is_split<kSlots>(p) && l == p.L - 1 ? (int)blockIdx.x % p.out_chunks : c;
+        if (++c == layer_chunks<kSlots>(p, l)) {
             c = 0;
             if (++l == p.L) l = 0, i += 2;
         }
@@ -252,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
     tc::tc_fence_after();
     const uint32_t taddr = *s_tmem;
     // this CTA's tiles are blockIdx.x + i gridDim.x, i < my_tiles (JobOrder deals them to the slots)
-    const int my_tiles = p.split ? 1 : (p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int my_tiles = is_split<kSlots>(p) ? 1 : (p.n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
     if (warp == kEpiWarps && lane == 0) {
         // ---------------- TMA producer ----------------
@@ -260,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
         uint32_t it = 0;
         SlotCount xc;
         bool ok = true;
-        JobOrder jobs(my_tiles);
+        JobOrder<kSlots> jobs(my_tiles);
         int s, t, l, c;
         while (ok && jobs.next(p, s, t, l, c)) {
             const int n = layer_n(p, l), nk = layer_kblocks(p, l);
@@ -290,14 +301,14 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
         SlotCount ja, xm, hw;
         bool ok = true;
         const uint32_t idesc_h = tc::idesc_bf16(128, p.hidden), idesc_o = tc::idesc_bf16(128, 256);
-        JobOrder jobs(my_tiles);
+        JobOrder<kSlots> jobs(my_tiles);
         int s, t, l, c;
         while (ok && jobs.next(p, s, t, l, c)) {
-            const int nk = layer_kblocks(p, l), nc = layer_chunks(p, l);
+            const int nk = layer_kblocks(p, l), nc = layer_chunks<kSlots>(p, l);
             const uint32_t idesc = l < p.L - 1 ? idesc_h : idesc_o;
             if (!(ok = tc::mbar_wait(acc_empty + 8 * s, (ja.get(s) & 1) ^ 1, p.err))) break;
             if (l == 0) ok = tc::mbar_wait(x_full + 8 * s, xm.take(s) & 1, p.err);
-            else if (p.split || c == 0) ok = tc::mbar_wait(h_full + 8 * s, hw.take(s) & 1, p.err);
+            else if (is_split<kSlots>(p) || c == 0) ok = tc::mbar_wait(h_full + 8 * s, hw.take(s) & 1, p.err);
             if (!ok || *s_abort) { ok = false; break; }
             tc::tc_fence_after();
             const uint32_t d = taddr + 256u * s, a0 = sH + s * kHBytes;
@@ -313,7 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
             }
             if (!ok) break;
             // the slot's last MMAs of this tile: its activations may take the next X tile
-            if (l == p.L - 1 && (p.split || c == nc - 1)) tc::umma_commit(x_empty + 8 * s);
+            if (l == p.L - 1 && (is_split<kSlots>(p) || c == nc - 1)) tc::umma_commit(x_empty + 8 * s);
             tc::umma_commit(acc_full + 8 * s);
             ja.take(s);
         }
@@ -331,7 +342,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_forward_kernel(const __grid_c
         SlotCount je;
         int obuf = 0;
         bool ok = true;
-        JobOrder jobs(my_tiles);
+        JobOrder<kSlots> jobs(my_tiles);
         int s, t, l, c;
         while (ok && jobs.next(p, s, t, l, c)) {
             const bool hidden_l = l < p.L - 1;
