@@ -185,13 +185,14 @@ extern "C" int xmc_run_noalloc(const InputInfo* input, const xmc_options* opt, u
     size_t o_runs = 0, o_tail = 0, o_clear = 0;
     if (kp.coop_query && room(b_runs, &o_runs)) kp.cell_runs = reinterpret_cast<const uint32_t*>(scratch + o_runs);
     else kp.coop_query = 0;
-    // The tail kernel, with a list for what the transport kernel's warps hand over, or for runs of up to half as many
-    // photons as the grid has threads, which it walks whole. 4e4 / 6e4 photons lost at the Area's faces, whole and
-    // through both kernels: ellipsoid of 1,280 triangles 13.5 / 16.5 and 12.9 / 13.4 ms, planar stack 2.9 / 3.7 and
-    // 2.4 / 2.5; 3e4 photons, ellipsoid of 5,120: 14.4 and 17.2.
+    // The tail kernel, with a list for what the transport kernel's warps hand over, or for runs that it walks whole: up to
+    // half as many photons as the grid has threads, with no clearance grid (kClearanceRun). Ellipsoid of 1,280
+    // triangles, 4e4 / 6e4 photons, whole and through both kernels: 13.5 / 16.5 and 12.9 / 13.4 ms; of 5,120, 3e4
+    // photons: 14.4 and 17.2.
     int tail_occ = 0, tail_photons = 0;
     NA_CK(tail_occupancy(kp, &c.tail_smem, &tail_occ, &tail_photons));
-    c.tail_takes_small_runs = n_photons <= (unsigned long long)c.grid * c.block / 2;
+    const uint64_t threads = (uint64_t)c.grid * c.block;
+    c.tail_takes_small_runs = n_photons <= std::min(threads / 2, whole_in_tail_max(kp, threads));
     const size_t b_tail = c.tail_takes_small_runs ? 0 : sizeof(TailPhoton) * (size_t)c.grid * (c.block / 32) * kTailLanes;
     if (tail_occ > 0 && room(b_tail, &o_tail)) {
         c.tail_grid = sms * tail_occ;

@@ -599,10 +599,7 @@ template <bool kBias, bool kLog>
 static cudaError_t enqueue_variant(Context* ctx) {
     KParams kp = ctx->kp;
     const cudaStream_t st = ctx->stream;
-    // A run of fewer photons than the transport grid has threads would leave every warp thin from the start:
-    // the tail kernel takes it whole (2e4 photons: 2.5 ms through both kernels, 1.75 ms this way; 6e4: 12.9
-    // and 10.2 ms).
-    kp.tail_direct = kp.tail && ctx->tail_takes_small_runs && kp.n_photons <= (unsigned long long)ctx->grid * ctx->block;
+    kp.tail_direct = kp.tail && ctx->tail_takes_small_runs && kp.n_photons <= whole_in_tail_max(kp, (uint64_t)ctx->grid * ctx->block);
     if (kp.tail_direct) ++g_debug_counts.whole_in_tail;
     if (kp.tail) {
         const cudaError_t e = cudaMemsetAsync(kp.tail_count, 0, 2 * sizeof(unsigned), st);

@@ -368,6 +368,20 @@ void build_xy_grid(const GeomImage& g, GridImage* out, int tris_per_cell = 2, co
 // bvh.cpp: clearance grid of the triangles of `g` that are neither big in `grid` nor horizontal; fills kp's clearance fields
 void build_clearance(const GeomImage& g, const GridImage& grid, KParams* kp, std::vector<uint8_t>* clear);
 
+// Most photons of a run that the tail kernel walks whole, on a grid of `threads` transport threads. Few photons leave
+// every warp of the transport kernel thin from the start; the more of them, and the shorter their walks beside
+// the longest one, the more its warps are worth. Where the two meet (75,776 threads; ms whole / through both kernels):
+// biased walks at the threads themselves (75,000: 3.8 / 3.8); walks that no Area face ends at four fifths
+// (60,000: planar stack 9.0 / 9.4, glass cover 9.1 / 8.1, height field 11.9 / 12.0, ellipsoid 15.5 / 16.4); of the others, those
+// in a mesh at three fifths (37,000 and 50,000: height field 6.4 / 5.9 and 7.6 / 6.1, ellipsoid 8.8 / 10.4
+// and 11.2 / 10.9), those in a stack of planes at a third (25,000: 2.3 / 2.3, glass
+// cover 2.2 / 2.3; 75,000: 4.4 / 2.7).
+inline uint64_t whole_in_tail_max(const KParams& kp, uint64_t threads) {
+    if (kp.use_bias) return threads;
+    if (kp.flags & XMC_NO_AREA_KILL) return threads * 4 / 5;
+    return kp.n_tris > kMaxBigTriangles ? threads * 3 / 5 : threads / 3;
+}
+
 // transport.cu: enqueue one transport kernel launch on ctx->stream (tallies must be zeroed).
 cudaError_t enqueue_transport(Context* ctx);
 // sparse_maps.cu: blocks of cells per map, and the two passes of the sparse map read-back
