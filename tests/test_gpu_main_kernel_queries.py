@@ -80,3 +80,41 @@ def test_maps_of_the_transport_kernel_agree_with_the_replay(tmp_path, log):
     for k in got[0][0]:
         assert np.array_equal(got[0][0][k], got[1][0][k]), k
     assert np.array_equal(got[0][1], got[1][1])
+
+
+def _stack():
+    """Four height fields 0.2 mm apart: a walk among triangles wherever it goes, so that warps take rounds in which
+    every lane takes the general step."""
+    sc = scenes.height_field_tissue(grid=33, n_rings=10, time_bins=5)
+    top, upper, lower, bottom = sc.surfaces
+    sc.surfaces = [top, upper] + [scenes.height_field(0.25 + 0.2 * i, 0.09, 2.0, 33, 10.0) for i in range(4)] + [lower, bottom]
+    a, l1, l2, l3 = sc.layers
+    inner = [scenes.Layer(l2.n, l2.mua, l2.mus, l2.g, [s, s + 1]) for s in range(1, 6)]
+    sc.layers = [scenes.Layer(a.n, 0, 0, 0, [0, 7]), scenes.Layer(l1.n, l1.mua, l1.mus, l1.g, [0, 1])] + inner + \
+                [scenes.Layer(l3.n, l3.mua, l3.mus, l3.g, [6, 7])]
+    return sc
+
+
+@pytest.mark.parametrize("maps", [False, True])
+def test_rounds_of_general_steps_change_nothing(tmp_path, maps):
+    """The tail kernel has no such rounds: pieces of a run that it walks whole add up to the run."""
+    m = api.Model(*_stack().write(str(tmp_path), "stack"))
+    t = api.Transport(m, roulette=True, scattering=maps, trajectories=maps, **SHAPE)
+    n, piece = 40_000, 10_000
+    before = _whole_in_tail()
+    led = t.run(n, seed=31)
+    whole, maps_whole = t.tallies(), t.maps()
+    assert _whole_in_tail() == before
+    steps, total, maps_total = 0, None, None
+    for first in range(0, n, piece):
+        steps += t.run(piece, seed=31, first_photon=first)["steps"]
+        tal, mp = t.tallies(), t.maps()
+        total = tal if total is None else {k: total[k] + tal[k] for k in tal}
+        maps_total = mp if maps_total is None else {k: maps_total[k] + mp[k] for k in mp}
+    assert _whole_in_tail() - before >= n // piece  # (and replays)
+    t.close()
+    assert steps == led["steps"] and led["n_detected"] > 100
+    for k in whole:
+        assert np.array_equal(whole[k], total[k]), k
+    for k in maps_whole:
+        assert np.array_equal(maps_whole[k], maps_total[k]), k

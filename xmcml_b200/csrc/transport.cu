@@ -212,6 +212,14 @@ __device__ __forceinline__ void warp_grid_query(const KParams& P, WarpQuery& W, 
 
 }  // namespace
 
+// A warp among triangles wherever it goes (a stack of height fields) finds a batch of waiting lanes in its first free
+// step; trying it is then all loss. After kCrowdedRounds such rounds on end it takes kGeneralRounds of general
+// steps with every lane, then tries once more. Four height fields in a stack, 1e6 photons, ms without and with this:
+// 65 x 65 vertices 102 and 97, 257 x 257 118 and 112, 17 x 17 83 and 77 (every step general: 96, 113, 72); elsewhere it
+// hardly happens (height field 38.7 and 38.6, ellipsoid 48.1 and 48.2, glass cover 12.75 and 12.95). Taken at the first
+// crowded round it cost the glass cover 5 to 40 %. Not for the biased walk (18.9 and 19.4).
+constexpr int kCrowdedRounds = 6, kGeneralRounds = 32;
+
 // kBias: biased spin with 64-bit weights; kLog: run pass that logs crossings for the trajectory maps
 template <bool kBias, bool kLog>
 __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
@@ -254,6 +262,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
     unsigned xn = 0;  // crossings of the current photon (capacity + 1: the log overflowed)
     unsigned long long cbeg = 0, cend = 0;  // warp-uniform chunk of photon indices
     bool exhausted = false;                 // warp-uniform
+    int general = 0;                        // warp-uniform: general rounds to come, or less the crowded ones just seen
     bool alive = false;
     Photon<WT> ph;
     ph.rdet = -1;
@@ -361,9 +370,10 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
         // ---- free steps of every lane, until enough lanes wait for the general step below: a query, glass, a
         // photon lost at the Area's faces, cut or at its step budget ----
         const int batch = exhausted ? max(1, min(P.query_batch, __popc(living) / 4)) : P.query_batch;
-        bool wait = false;
-        unsigned waiting;
+        bool wait = general > 0 && alive;
+        unsigned waiting = 0u, before;
         do {
+            before = waiting;
             if (alive && !wait) {
                 const uint4 r = philox4x32_10(make_uint4((uint32_t)ph.pid, (uint32_t)(ph.pid >> 32), ph.iter, 0u), P.keys);
                 const DevLayer& L = s_layer[ph.layer];
@@ -395,6 +405,11 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
             }
             waiting = __ballot_sync(FULL, wait);
         } while (__popc(waiting) < batch && waiting != (kBias ? __ballot_sync(FULL, alive) : living));
+
+        if (!kBias) {
+            if (general > 0) general = general == 1 ? 1 - kCrowdedRounds : general - 1;
+            else general = before != 0u ? 0 : general == 1 - kCrowdedRounds ? kGeneralRounds : general - 1;
+        }
 
         // ---- one walk iteration of the waiting lanes (mcml_kernel.cpp:47-125) ----
         // Up to the ray query no lane leaves the iteration, so that every lane reaches the query
