@@ -491,7 +491,7 @@ def measure_batch(args, rank, world, local, dist, torch, barrier, n_steps, n_war
                     "l2": "instance table re-uploaded and 24.6 MB of tallies zeroed every step"},
             "clocks": clocks,
             "e2e": {"value": world * n_steps * total / wall_s, "unit": UNIT,
-                    "h2d_bytes_per_step": K * (32 + 5 * 48), "d2h_bytes_per_step": K * (R * T * 8 + R * 8 + 16 * 8) + 4,
+                    "h2d_bytes_per_step": K * (40 + 5 * 48) + 24, "d2h_bytes_per_step": K * (R * T * 8 + R * 8 + 16 * 8) + 4,
                     "via": "xmc_batch_run with host instance table and host result arrays"},
             "gpu_launches": 3 * n_steps, "roofline": rl, "cpu_baseline": cpu,
             "walk": {"steps_per_photon": steps / total}}

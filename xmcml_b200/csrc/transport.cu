@@ -14,8 +14,8 @@
 // their own, until P.query_batch lanes wait for a general step; then it takes those together: one
 // cooperative ray query, boundary optics, detection and deaths. Which lanes take a step together changes no
 // photon's path. B200, ps per step at 1e6 photons and more, every step general -> free steps apart, with
-// the clearance grid and the wider cell rectangles: planar stack with roulette 28.0 -> 18.7, height field
-// 34.7 -> 27.3, ellipsoid 87.6 -> 73.3, glass cover 46.4 -> 40.5. What bounds it now is instruction issue
+// the clearance grid, the wider cell rectangles and no branches in the free step: planar stack with roulette 28.0 ->
+// 17.6, height field 34.7 -> 25.7, ellipsoid 87.6 -> 72.5, glass cover 46.4 -> 40.6. What bounds it now is instruction issue
 // (about 300 per free iteration of the warp, 17 of 32 lanes active on average) at 16 warps per SM.
 //
 // Per iteration (tissue layer): slot 0 step length; on a boundary hit slot 1 Fresnel test and

@@ -1,5 +1,5 @@
 // Photon state and the steps of the walk shared by the transport kernel (one photon per thread) and the
-// tail kernel (one photon per warp): voxel index, detector search and tallies, plane crossings, launch,
+// tail kernel (one photon per group of 8 lanes): voxel index, detector search and tallies, plane crossings, launch,
 // boundary crossing and the biased spin. Both kernels inline the same arithmetic, so a photon takes the
 // same path in either.
 #pragma once
