@@ -14,8 +14,8 @@
 // their own, until P.query_batch lanes wait for a general step; then it takes those together: one
 // cooperative ray query, boundary optics, detection and deaths. Which lanes take a step together changes no
 // photon's path. B200, ps per step at 1e6 photons and more, every step general -> free steps apart, with
-// the clearance grid, the wider cell rectangles and no branches in the free step: planar stack with roulette 28.0 ->
-// 17.6, height field 34.7 -> 25.7, ellipsoid 87.6 -> 72.5, glass cover 46.4 -> 40.6. What bounds it now is instruction issue
+// the clearance grid and the wider cell rectangles: planar stack with roulette 28.0 -> 18.7, height field
+// 34.7 -> 27.3, ellipsoid 87.6 -> 73.3, glass cover 46.4 -> 40.5. What bounds it now is instruction issue
 // (about 300 per free iteration of the warp, 17 of 32 lanes active on average) at 16 warps per SM.
 //
 // Per iteration (tissue layer): slot 0 step length; on a boundary hit slot 1 Fresnel test and
@@ -218,7 +218,14 @@ __device__ __forceinline__ void warp_grid_query(const KParams& P, WarpQuery& W, 
 // 65 x 65 vertices 102 and 97, 257 x 257 118 and 112, 17 x 17 83 and 77 (every step general: 96, 113, 72); elsewhere it
 // hardly happens (height field 38.7 and 38.6, ellipsoid 48.1 and 48.2, glass cover 12.75 and 12.95). Taken at the first
 // crowded round it cost the glass cover 5 to 40 %. Not for the biased walk (18.9 and 19.4).
-constexpr int kCrowdedRounds = 6, kGeneralRounds = 32;
+constexpr int kCrowdedRounds = 6, kGeneralRounds = 32, kExhausted = -1000;
+
+// Whether a warp has no photons left to claim. The variant with logs has no register for a word of its own (1.4 % of a
+// height field with every map): there it takes the place of `general`, and no more general rounds are made.
+template <bool kLog>
+__device__ __forceinline__ bool out_of_ids(int general, bool no_ids) {
+    return kLog ? general == kExhausted : no_ids;
+}
 
 // kBias: biased spin with 64-bit weights; kLog: run pass that logs crossings for the trajectory maps
 template <bool kBias, bool kLog>
@@ -261,8 +268,8 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
     const bool record_planes = P.mode == 1 || (P.flags & XMC_SCATTERING_MAP) != 0 || log_traj;
     unsigned xn = 0;  // crossings of the current photon (capacity + 1: the log overflowed)
     unsigned long long cbeg = 0, cend = 0;  // warp-uniform chunk of photon indices
-    bool exhausted = false;                 // warp-uniform
     int general = 0;                        // warp-uniform: general rounds to come, or less the crowded ones just seen
+    bool no_ids = false;                    // warp-uniform: no photons are left to claim (out_of_ids)
     bool alive = false;
     Photon<WT> ph;
     ph.rdet = -1;
@@ -314,7 +321,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
             }
         }
         // ---- refill dead lanes with new photons (warp-level compaction) ----
-        unsigned need = __ballot_sync(FULL, !alive && !exhausted);
+        unsigned need = __ballot_sync(FULL, !alive && !out_of_ids<kLog>(general, no_ids));
         while (need) {
             if (cbeg == cend) {
                 unsigned long long b = 0;
@@ -327,7 +334,8 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
                 cancelled = __shfl_sync(FULL, cancelled, 0);
                 if (cancelled && lane == 0) atomicOr(P.status, 2);
                 if (b >= P.n_photons) {
-                    exhausted = true;
+                    if constexpr (kLog) general = kExhausted;
+                    else no_ids = true;
                     break;
                 }
                 cbeg = b;
@@ -352,12 +360,12 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
                 atomicAdd(&S.ledger[L_LAUNCHED], 1ull);
             }
             cbeg += take;
-            need = __ballot_sync(FULL, !alive && !exhausted);
+            need = __ballot_sync(FULL, !alive && !out_of_ids<kLog>(general, no_ids));
         }
         const unsigned living = __ballot_sync(FULL, alive);
         if (living == 0u) break;
         // ---- no photons left to claim and few left in the warp: they go to the tail kernel ----
-        if (exhausted && P.tail && __popc(living) <= kTailLanes) {
+        if (out_of_ids<kLog>(general, no_ids) && P.tail && __popc(living) <= kTailLanes) {
             if (alive) {
                 steps -= ph.iter;  // the tail kernel counts the whole walk
                 unsigned xrow = 0;
@@ -369,7 +377,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
 
         // ---- free steps of every lane, until enough lanes wait for the general step below: a query, glass, a
         // photon lost at the Area's faces, cut or at its step budget ----
-        const int batch = exhausted ? max(1, min(P.query_batch, __popc(living) / 4)) : P.query_batch;
+        const int batch = out_of_ids<kLog>(general, no_ids) ? max(1, min(P.query_batch, __popc(living) / 4)) : P.query_batch;
         bool wait = general > 0 && alive;
         unsigned waiting = 0u, before;
         do {
@@ -406,7 +414,7 @@ __global__ void __launch_bounds__(512, 1) transport_kernel(const KParams P) {
             waiting = __ballot_sync(FULL, wait);
         } while (__popc(waiting) < batch && waiting != (kBias ? __ballot_sync(FULL, alive) : living));
 
-        if (!kBias) {
+        if (!kBias && (!kLog || general != kExhausted)) {
             if (general > 0) general = general == 1 ? 1 - kCrowdedRounds : general - 1;
             else general = before != 0u ? 0 : general == 1 - kCrowdedRounds ? kGeneralRounds : general - 1;
         }
